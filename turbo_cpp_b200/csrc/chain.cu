@@ -135,11 +135,14 @@ struct DevTb {
   int64_t bits_out;  // offset of the block's TBS output bits
 };
 
-// Per code block of a transport-block call: its transport block and where its kept bits start in
-// that block's TBS + CRC24A stream (the sum of the kept bits of the blocks before it).
+// Per code block of a transport-block call: its transport block, where its kept bits start in
+// that block's TBS + CRC24A stream (the sum of the kept bits of the blocks before it), its size
+// and filler and the float offset of its posterior.
 struct DevTbCb {
   int32_t tb;
   int32_t pos;
+  int32_t k, filler;
+  int64_t out;
 };
 
 constexpr int kFinishThreads = 256;
@@ -151,7 +154,7 @@ constexpr int kFinishThreads = 256;
 // x^(N-1-j) mod g over the set bits j of the N-bit codeword, so the shares of a transport
 // block's code blocks XOR to its syndrome.
 __global__ void __launch_bounds__(kFinishThreads) tb_finish_cb_kernel(
-    const DevTb* __restrict__ tbs, const DevTbCb* __restrict__ tbcb, const DevCb* __restrict__ cbs,
+    const DevTb* __restrict__ tbs, const DevTbCb* __restrict__ tbcb,
     const float* __restrict__ post, const uint32_t* __restrict__ xpow_a,
     const uint32_t* __restrict__ xpow_b, uint8_t* __restrict__ bits, uint8_t* __restrict__ cb_ok,
     uint32_t* __restrict__ syn_a_part) {
@@ -166,13 +169,12 @@ __global__ void __launch_bounds__(kFinishThreads) tb_finish_cb_kernel(
     return;
   }
   const DevTb t = tbs[m.tb];
-  const DevCb cb = cbs[c];
   const int64_t n_a = t.tbs + 24;             // TB codeword length with CRC24A
-  const int n_b = cb.k - cb.filler;           // CRC24B codeword length
+  const int n_b = m.k - m.filler;             // CRC24B codeword length
   const int keep = n_b - (t.n_cb > 1 ? 24 : 0);
   uint32_t syn_b = 0, syn_a = 0;
   for (int i = threadIdx.x; i < n_b; i += kFinishThreads) {
-    const uint8_t bit = post[cb.out + cb.filler + i] >= 0.0f ? 1 : 0;
+    const uint8_t bit = post[m.out + m.filler + i] >= 0.0f ? 1 : 0;
     if (bit) syn_b ^= xpow_b[n_b - 1 - i];
     if (i < keep) {
       const int64_t j = m.pos + i;
@@ -205,7 +207,7 @@ __global__ void __launch_bounds__(kFinishThreads) tb_finish_cb_kernel(
 // Finish, part 2, one thread per transport block: the XOR of its code blocks' CRC24A shares,
 // and whether the kept bits add up to TBS + 24.
 __global__ void tb_finish_tb_kernel(const DevTb* __restrict__ tbs, int n_tb,
-                                    const DevTbCb* __restrict__ tbcb, const DevCb* __restrict__ cbs,
+                                    const DevTbCb* __restrict__ tbcb,
                                     const uint32_t* __restrict__ syn_a_part,
                                     uint8_t* __restrict__ tb_ok) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -213,9 +215,8 @@ __global__ void tb_finish_tb_kernel(const DevTb* __restrict__ tbs, int n_tb,
   const DevTb d = tbs[t];
   uint32_t a = 0;
   for (int r = 0; r < d.n_cb; ++r) a ^= syn_a_part[d.first_cb + r];
-  const int last = d.first_cb + d.n_cb - 1;
-  const DevCb cb = cbs[last];
-  const int64_t kept_end = tbcb[last].pos + cb.k - cb.filler - (d.n_cb > 1 ? 24 : 0);
+  const DevTbCb last = tbcb[d.first_cb + d.n_cb - 1];
+  const int64_t kept_end = last.pos + last.k - last.filler - (d.n_cb > 1 ? 24 : 0);
   tb_ok[t] = (kept_end == d.tbs + 24) && a == 0;
 }
 
@@ -382,14 +383,18 @@ void Decoder::transport_blocks(const TbRequest& q, bool wait, void* after, void*
   }
   // per code block: its transport block and the start of its kept bits in that block's stream
   // (a block that belongs to no transport block keeps tb = -1: decoded, then left out)
-  std::vector<DevTbCb> tbcb(q.n_cb, DevTbCb{-1, 0});
+  std::vector<DevTbCb> tbcb(q.n_cb);
+  for (size_t i = 0; i < q.n_cb; ++i)
+    tbcb[i] = DevTbCb{-1, 0, cbs[i].k, cbs[i].filler, cbs[i].out_offset};
   for (size_t t = 0; t < q.n_tb; ++t) {
     int64_t pos = 0;
     for (int r = 0; r < tbs[t].n_cb; ++r) {
       const auto& c = q.cbs[tbs[t].first_cb + r];
       if (tbcb[tbs[t].first_cb + r].tb >= 0)
         throw InvalidArgument("a code block belongs to two transport blocks");
-      tbcb[tbs[t].first_cb + r] = DevTbCb{static_cast<int32_t>(t), static_cast<int32_t>(pos)};
+      DevTbCb& m = tbcb[tbs[t].first_cb + r];
+      m.tb = static_cast<int32_t>(t);
+      m.pos = static_cast<int32_t>(pos);
       pos += c.k - c.filler - (tbs[t].n_cb > 1 ? 24 : 0);
     }
   }
@@ -441,16 +446,15 @@ void Decoder::transport_blocks(const TbRequest& q, bool wait, void* after, void*
   if (rq.auto_schedule) rq = resolve_locked(rq);  // the tuning table's schedule and window
   auto body = [&] {
     derate_device(q.n_cb, rm.data(), e_llr, q.e_len, d012, static_cast<size_t>(llr_len), st);
-    if (rq.persistent) decode_persistent(rq); else decode_plain(rq);
-    // decode_* chained its own completion event; the finish kernel follows on the same stream
+    decode_now(rq);
+    // decode_now chained its own completion event; the finish kernel follows on the same stream
     upload(dtb, tbs.data(), q.n_tb * sizeof(DevTb), st);
     upload(dtbcb, tbcb.data(), q.n_cb * sizeof(DevTbCb), st);
-    const DevCb* dcbs = static_cast<const DevCb*>(d_cbs_.ptr);
     tb_finish_cb_kernel<<<static_cast<unsigned>(q.n_cb), kFinishThreads, 0, st>>>(
-        dtb, dtbcb, dcbs, post, static_cast<const uint32_t*>(xpow_a.ptr),
+        dtb, dtbcb, post, static_cast<const uint32_t*>(xpow_a.ptr),
         static_cast<const uint32_t*>(std3gpp ? d_xpow_std_.ptr : d_xpow_.ptr), bits, cb_ok, dsyn);
     tb_finish_tb_kernel<<<static_cast<unsigned>((q.n_tb + 255) / 256), 256, 0, st>>>(
-        dtb, static_cast<int>(q.n_tb), dtbcb, dcbs, dsyn, tb_ok);
+        dtb, static_cast<int>(q.n_tb), dtbcb, dsyn, tb_ok);
     check(cudaGetLastError(), "finish launch");
     timing_.launches += 2;
     if (q.device_memory && q.posterior)
@@ -469,7 +473,7 @@ void Decoder::transport_blocks(const TbRequest& q, bool wait, void* after, void*
     const int64_t opts[9] = {static_cast<int64_t>(q.n_tb), static_cast<int64_t>(q.n_cb),
                              static_cast<int64_t>(q.e_len), static_cast<int64_t>(q.bits_len),
                              rq.max_iterations, rq.early_stop, rq.window, rq.guard,
-                             (rq.std3gpp ? 4 : 0) | (rq.persistent ? 2 : 0) | (rq.smem_checkpoints ? 1 : 0)};
+                             (rq.std3gpp ? 4 : 0) | (rq.persistent ? 2 : 0)};
     put(ptrs, sizeof ptrs);
     put(opts, sizeof opts);
     put(rm.data(), q.n_cb * sizeof(RmBlockDesc));

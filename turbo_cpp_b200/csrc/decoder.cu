@@ -1,10 +1,12 @@
-// decoder.cu -- the plain (host-driven) GPU turbo decoder and its device buffers.
+// decoder.cu -- the GPU turbo decoder and its device buffers.
 //
-// One tc_decode call decodes any number of code blocks of any LTE sizes.  Per full iteration
-// the host enqueues two launches (upper SISO over natural order, lower SISO over QPP order) and,
-// with early stop, one CRC24B launch; every thread owns one window of one code block.  This is
-// the replacement of the reference's Stage 1/2 host loops (lte_turbo_cuda.cu:1391-1540,
-// 1719-1899), batched over code blocks and correct for every K.
+// One tc_decode call decodes any number of code blocks of any LTE sizes; every thread owns one
+// window of one code block.  The block-resident kernel (resident.cuh) runs all iterations in one
+// launch; layouts it cannot hold (very long windows in large batches, more than 256 windows per
+// block, more than 64 iterations) run as two launches per iteration (upper SISO over natural
+// order, lower SISO over QPP order) and, with early stop, one CRC24B launch.  This is the
+// replacement of the reference's Stage 1/2 host loops (lte_turbo_cuda.cu:1391-1540, 1719-1899),
+// batched over code blocks and correct for every K.
 #include <cuda_runtime.h>
 
 #include <functional>
@@ -23,10 +25,28 @@
 #include "decoder.hpp"
 #include "lte_codec.hpp"
 #include "decode_kernels.cuh"
+#include "resident.cuh"
 
 namespace tcb {
 
 namespace {
+
+// The kernel instances: CTAs of 32, 64, 96, 128 or 256 threads.
+constexpr int kResThreads[] = {32, 64, 96, 128, 256};
+using ResKernel = void (*)(ResArgs);
+template <bool STD>
+ResKernel res_kernel_of(int threads) {
+  switch (threads) {
+    case 32: return resident_kernel<STD, 32>;
+    case 64: return resident_kernel<STD, 64>;
+    case 96: return resident_kernel<STD, 96>;
+    case 128: return resident_kernel<STD, 128>;
+    default: return resident_kernel<STD, 256>;
+  }
+}
+ResKernel res_kernel(bool std3gpp, int threads) {
+  return std3gpp ? res_kernel_of<true>(threads) : res_kernel_of<false>(threads);
+}
 
 void check(cudaError_t e, const char* what) {
   if (e != cudaSuccess)
@@ -108,63 +128,48 @@ Decoder::Decoder(int device) : device_(device) {
     }
     inv.insert(inv.end(), iv.begin(), iv.end());
   }
-  // x^j mod g_CRC24B for j < 6144
-  std::vector<uint32_t> xpow(6144);
-  const uint32_t g = crc_generator_mask(CrcKind::Crc24B);
-  uint32_t r = 1;
-  for (int j = 0; j < 6144; ++j) {
-    xpow[j] = r;
-    r <<= 1;
-    if (r & (1u << 24)) r ^= (1u << 24) | g;
-  }
   d_perm_.reserve(perm.size() * 2);
   d_inv_.reserve(inv.size() * 2);
-  d_xpow_.reserve(xpow.size() * 4);
   check(cudaMemcpy(d_perm_.ptr, perm.data(), perm.size() * 2, cudaMemcpyHostToDevice), "upload perm");
   check(cudaMemcpy(d_inv_.ptr, inv.data(), inv.size() * 2, cudaMemcpyHostToDevice), "upload inv");
-  check(cudaMemcpy(d_xpow_.ptr, xpow.data(), xpow.size() * 4, cudaMemcpyHostToDevice), "upload crc");
-  {  // the same for TS 36.212's CRC24B
-    const uint32_t gs = crc_generator_mask(CrcKind::Crc24B, Convention::Std3gpp);
-    uint32_t q = 1;
-    for (int j = 0; j < 6144; ++j) {
-      xpow[j] = q;
-      q <<= 1;
-      if (q & (1u << 24)) q ^= (1u << 24) | gs;
+  // x^j mod g_CRC24B for j < kXpowSize, then b(x) x^24 mod g for every byte b, in both conventions
+  for (const Convention conv : {Convention::Reference, Convention::Std3gpp}) {
+    std::vector<uint32_t> xpow(kXpowSize + 256, 0);
+    const uint32_t g = crc_generator_mask(CrcKind::Crc24B, conv);
+    uint32_t r = 1;
+    for (int j = 0; j < kXpowSize; ++j) {
+      xpow[j] = r;
+      r <<= 1;
+      if (r & (1u << 24)) r ^= (1u << 24) | g;
     }
-    d_xpow_std_.reserve(xpow.size() * 4);
-    check(cudaMemcpy(d_xpow_std_.ptr, xpow.data(), xpow.size() * 4, cudaMemcpyHostToDevice),
-          "upload crc");
+    for (int b = 0; b < 256; ++b)
+      for (int i = 0; i < 8; ++i)
+        if ((b >> i) & 1) xpow[kXpowSize + b] ^= xpow[24 + i];
+    DeviceBuffer& d = conv == Convention::Std3gpp ? d_xpow_std_ : d_xpow_;
+    d.reserve(xpow.size() * 4);
+    check(cudaMemcpy(d.ptr, xpow.data(), xpow.size() * 4, cudaMemcpyHostToDevice), "upload crc");
   }
   d_err_.reserve(sizeof(int));
   check(cudaMemset(d_err_.ptr, 0, sizeof(int)), "zero error word");
 
-  const int smem = smem_optin_;
-  for (const void* f : {reinterpret_cast<const void*>(siso_plain_kernel<kSub, 0, false>),
-                        reinterpret_cast<const void*>(siso_plain_kernel<kSub, 1, false>),
-                        reinterpret_cast<const void*>(siso_plain_kernel<kSub, 2, false>),
-                        reinterpret_cast<const void*>(siso_plain_kernel<kSub, 0, false, true>),
-                        reinterpret_cast<const void*>(siso_plain_kernel<kSub, 1, false, true>),
-                        reinterpret_cast<const void*>(siso_plain_kernel<kSub, 2, false, true>)})
-    check(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "smem attr");
-  for (const void* f : {reinterpret_cast<const void*>(siso_plain_kernel<kSub, 0, true>),
+  for (const void* f : {reinterpret_cast<const void*>(siso_plain_kernel<kSub, 0>),
+                        reinterpret_cast<const void*>(siso_plain_kernel<kSub, 1>),
+                        reinterpret_cast<const void*>(siso_plain_kernel<kSub, 2>),
+                        reinterpret_cast<const void*>(siso_plain_kernel<kSub, 0, true>),
                         reinterpret_cast<const void*>(siso_plain_kernel<kSub, 1, true>),
-                        reinterpret_cast<const void*>(siso_plain_kernel<kSub, 2, true>),
-                        reinterpret_cast<const void*>(siso_plain_kernel<kSub, 0, true, true>),
-                        reinterpret_cast<const void*>(siso_plain_kernel<kSub, 1, true, true>),
-                        reinterpret_cast<const void*>(siso_plain_kernel<kSub, 2, true, true>),
-                        reinterpret_cast<const void*>(persistent_kernel<false>),
-                        reinterpret_cast<const void*>(persistent_kernel<true>)})
+                        reinterpret_cast<const void*>(siso_plain_kernel<kSub, 2, true>)})
     check(cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 0),
           "carveout attr");
+  for (const int t : kResThreads)
+    for (const bool std3gpp : {false, true}) {
+      const ResKernel f = res_kernel(std3gpp, t);
+      check(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kResMaxSmem),
+            "smem attr");
+      check(cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                 cudaSharedmemCarveoutMaxShared),
+            "carveout attr");
+    }
   configure_chain_kernels();
-  int per_sm_std = 0;
-  check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_std, persistent_kernel<true>,
-                                                      kPersistThreads, 0),
-        "occupancy");
-  check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&persist_blocks_per_sm_, persistent_kernel<false>,
-                                                      kPersistThreads, 0),
-        "occupancy");
-  persist_blocks_per_sm_ = std::min(persist_blocks_per_sm_, per_sm_std);
 }
 
 Decoder::~Decoder() {
@@ -181,7 +186,7 @@ Decoder::~Decoder() {
   if (stream_) cudaStreamDestroy(static_cast<cudaStream_t>(stream_));
   for (DeviceBuffer* b : {&d_perm_, &d_inv_, &d_xpow_, &d_xpow_std_, &d_xpow_a_std_, &d_cbs_, &d_wincb_, &d_llr_,
                           &d_sysi_, &d_e1i_, &d_e2_, &d_post_, &d_seed_, &d_done_, &d_iters_,
-                          &d_crc_, &d_ckpt_, &d_tasks_, &d_queue_, &d_rm_, &d_e_llr_, &d_d012_,
+                          &d_crc_, &d_ckpt_, &d_queue_, &d_rescbs_, &d_rm_, &d_e_llr_, &d_d012_,
                           &d_tbpost_, &d_tbbits_, &d_tbok_, &d_cbok_, &d_tbiters_, &d_tb_, &d_tbcb_, &d_synpart_,
                           &d_xpow_a_, &d_rmgroup_, &d_gen_, &d_gentab_, &d_genenc_, &d_genrm_})
     b->release();
@@ -275,11 +280,6 @@ int32_t Decoder::table_offset(int32_t k) const {
   return tab_offset_[qi];
 }
 
-int Decoder::pick_window(int32_t k, int32_t requested) const {
-  if (requested > 0) return std::min<int32_t>(requested, k);
-  return std::min<int32_t>(kDefaultWindow, k);
-}
-
 void Decoder::decode(const DecodeRequest& rq_in) {
   const DecodeRequest rq = rq_in.auto_schedule ? resolve(rq_in) : rq_in;
   if (rq.graph && rq.device_memory && rq.n_cb > 0) {
@@ -291,10 +291,7 @@ void Decoder::decode(const DecodeRequest& rq_in) {
     decode_host_async(rq);
     return;
   }
-  if (rq.persistent)
-    decode_persistent(rq);
-  else
-    decode_plain(rq);
+  decode_now(rq);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -519,38 +516,81 @@ void Decoder::decode_graph(const DecodeRequest& rq) {
   const int64_t opts[8] = {static_cast<int64_t>(rq.n_cb), static_cast<int64_t>(rq.llr_len),
                            static_cast<int64_t>(rq.post_len), rq.max_iterations, rq.early_stop,
                            rq.window, rq.guard,
-                           (rq.std3gpp ? 4 : 0) | (rq.persistent ? 2 : 0) | (rq.smem_checkpoints ? 1 : 0)};
+                           (rq.std3gpp ? 4 : 0) | (rq.persistent ? 2 : 0)};
   put(ptrs, sizeof ptrs);
   put(opts, sizeof opts);
   put(rq.cbs, rq.n_cb * sizeof(CodeBlockDesc));
   if (rq.scales) put(rq.scales, 2 * rq.max_iterations * sizeof(float));
   DecodeRequest eager = rq;
   eager.graph = false;
-  GraphEntry* e = graph_for(key, rq.stream, [&] {
-    if (eager.persistent) decode_persistent(eager); else decode_plain(eager);
-  });
+  GraphEntry* e = graph_for(key, rq.stream, [&] { decode_now(eager); });
   launch_graph(e, rq.stream);
 }
 
+// ------------------------------------------------------------------------------------------
+// One decode
+// ------------------------------------------------------------------------------------------
+struct Decoder::Layout {
+  std::vector<DevCb> cbs;  // in the caller's order (win0, work: run_sweeps)
+  int guard = 0;
+  int max_window = 0;
+  int max_windows = 0;  // of a block
+  int64_t steps = 0;    // sum of K
+  // block-resident kernel: blocks in task order, first block of each task
+  bool resident = false;
+  std::vector<ResCb> res;
+  std::vector<int32_t> task_first;
+  int threads = 0;
+  size_t smem = 0;
+};
+
+struct Decoder::Io {
+  const float* llr;
+  float* post;
+  uint8_t* crc;
+  uint32_t* iters;
+};
+
 namespace {
-// one plain-schedule SISO launch: kind 0 upper, 1 lower, 2 lower + posterior
-template <bool STD>
-void launch_plain(int kind, bool global_ckpt, int blocks, size_t smem, cudaStream_t st,
-                  const DevCb* dcbs, const int32_t* dwin, int n_win, const SisoIo& io,
-                  const uint8_t* dn, float4* ckpt, int max_ckpt) {
-  if (global_ckpt) {
-    if (kind == 0) siso_plain_kernel<kSub, 0, true, STD><<<blocks, kThreads, 0, st>>>(dcbs, dwin, n_win, io, dn, ckpt, max_ckpt);
-    else if (kind == 1) siso_plain_kernel<kSub, 1, true, STD><<<blocks, kThreads, 0, st>>>(dcbs, dwin, n_win, io, dn, ckpt, max_ckpt);
-    else siso_plain_kernel<kSub, 2, true, STD><<<blocks, kThreads, 0, st>>>(dcbs, dwin, n_win, io, dn, ckpt, max_ckpt);
-  } else {
-    if (kind == 0) siso_plain_kernel<kSub, 0, false, STD><<<blocks, kThreads, smem, st>>>(dcbs, dwin, n_win, io, dn, nullptr, 0);
-    else if (kind == 1) siso_plain_kernel<kSub, 1, false, STD><<<blocks, kThreads, smem, st>>>(dcbs, dwin, n_win, io, dn, nullptr, 0);
-    else siso_plain_kernel<kSub, 2, false, STD><<<blocks, kThreads, smem, st>>>(dcbs, dwin, n_win, io, dn, nullptr, 0);
-  }
-}
+// Bytes of X (shared memory) of a task with `lanes` windows of up to `window` steps.
+size_t res_x_bytes(int lanes, int window) { return 4 * static_cast<size_t>(window) * res_pitch(lanes); }
+// and what stands in front of it
+size_t res_head_bytes(int threads) { return static_cast<size_t>(res_x_at(threads)); }
+
 }  // namespace
 
-void Decoder::decode_plain(const DecodeRequest& rq) {
+void Decoder::check_request(const DecodeRequest& rq) const {
+  if (reinterpret_cast<uintptr_t>(rq.llr) % 16 != 0)
+    throw InvalidArgument("the LLR buffer must be 16-byte aligned");
+  if (rq.persistent && rq.max_iterations > static_cast<uint32_t>(kMaxIterations))
+    throw InvalidArgument("max_iterations above 64");
+  const int guard = rq.guard < 0 ? kDefaultGuard : rq.guard;
+  if (guard % kGroup != 0) throw InvalidArgument("guard must be a multiple of 8");
+  for (size_t i = 0; i < rq.n_cb; ++i) {
+    const CodeBlockDesc& c = rq.cbs[i];
+    if (qpp_index(c.k) < 0) throw OutOfRange("unsupported QPP block size");
+    if (c.filler < 0 || c.filler >= c.k) throw InvalidArgument("invalid filler count");
+    if (c.llr_offset < 0 || c.llr_offset % 4 != 0 ||
+        static_cast<size_t>(c.llr_offset) + 3 * static_cast<size_t>(c.k + 4) > rq.llr_len)
+      throw InvalidArgument("invalid LLR offset (must be a multiple of 4 and in range)");
+    if (c.out_offset < 0 || static_cast<size_t>(c.out_offset) + static_cast<size_t>(c.k) > rq.post_len)
+      throw InvalidArgument("invalid posterior offset");
+    if (!rq.persistent) {
+      const int w = std::min<int32_t>(rq.window > 0 ? rq.window : kDefaultWindow, c.k);
+      if (w % kGroup != 0) throw InvalidArgument("window must be a multiple of 8");
+      if (guard > w && w < c.k) throw InvalidArgument("guard must not exceed the window");
+    }
+  }
+}
+
+uint64_t Decoder::decode_taped(const DecodeRequest& rq, const Tape& tape) {
+  std::lock_guard<std::mutex> lock(mu_);
+  const uint64_t before = timing_.launches;
+  decode_now(rq, &tape);
+  return timing_.launches - before;
+}
+
+void Decoder::decode_now(const DecodeRequest& rq, const Tape* tape) {
   check(cudaSetDevice(device_), "cudaSetDevice");
   // device memory: the caller's stream as given (NULL = legacy default stream, as in CUDA);
   // host memory: the caller's stream if given, else the decoder's own stream
@@ -558,137 +598,270 @@ void Decoder::decode_plain(const DecodeRequest& rq) {
                                                                : (rq.stream ? rq.stream : stream_));
   const size_t n = rq.n_cb;
   if (n == 0) return;
-
-  // ---- validate and lay out ----
-  if (reinterpret_cast<uintptr_t>(rq.llr) % 16 != 0)
-    throw InvalidArgument("the LLR buffer must be 16-byte aligned");
+  check_request(rq);
   order_after_previous(st);
-  const int guard = rq.guard < 0 ? kDefaultGuard : rq.guard;
-  if (guard % kGroup != 0) throw InvalidArgument("guard must be a multiple of 8");
-  std::vector<DevCb> cbs(n);
-  std::vector<int32_t> wincb;
-  int64_t work = 0;
-  int max_ckpt = 0;
+
+  // ---- windows of every block ----
+  Layout l;
+  l.guard = rq.guard < 0 ? kDefaultGuard : rq.guard;
+  l.cbs.resize(n);
   for (size_t i = 0; i < n; ++i) {
     const int32_t k = rq.cbs[i].k;
-    const int qi = qpp_index(k);
-    if (qi < 0) throw OutOfRange("unsupported QPP block size");
-    if (rq.cbs[i].filler < 0 || rq.cbs[i].filler >= k) throw InvalidArgument("invalid filler count");
-    if (rq.cbs[i].llr_offset < 0 || rq.cbs[i].llr_offset % 4 != 0 ||
-        static_cast<size_t>(rq.cbs[i].llr_offset) + 3 * static_cast<size_t>(k + 4) > rq.llr_len)
-      throw InvalidArgument("invalid LLR offset (must be a multiple of 4 and in range)");
-    if (rq.cbs[i].out_offset < 0 ||
-        static_cast<size_t>(rq.cbs[i].out_offset) + static_cast<size_t>(k) > rq.post_len)
-      throw InvalidArgument("invalid posterior offset");
-    DevCb& d = cbs[i];
+    DevCb& d = l.cbs[i];
     d.k = k;
     d.filler = rq.cbs[i].filler;
-    d.tab = tab_offset_[qi];
-    d.window = pick_window(k, rq.window);
-    if (d.window % kGroup != 0) throw InvalidArgument("window must be a multiple of 8");
-    if (guard > d.window && d.window < k) throw InvalidArgument("guard must not exceed the window");
+    d.tab = tab_offset_[qpp_index(k)];
+    if (rq.persistent) {  // at most 32 windows of >= `target` steps (a multiple of 8, >= guard)
+      const int target = rq.window > 0 ? rq.window : kPersistWindow;
+      int nwin = std::max(1, std::min(32, k / std::max(target, 8)));
+      int wlen = ((k + nwin - 1) / nwin + kGroup - 1) / kGroup * kGroup;
+      if (nwin > 1 && wlen < l.guard) {  // windows may not be shorter than the guard
+        nwin = std::max(1, k / l.guard);
+        wlen = ((k + nwin - 1) / nwin + kGroup - 1) / kGroup * kGroup;
+      }
+      d.window = std::min<int32_t>(wlen, k);
+    } else {
+      d.window = std::min<int32_t>(rq.window > 0 ? rq.window : kDefaultWindow, k);
+    }
     d.nwin = (k + d.window - 1) / d.window;
-    d.win0 = static_cast<int32_t>(wincb.size());
     d.llr = rq.cbs[i].llr_offset;
-    d.work = work;
+    d.work = l.steps;
     d.out = rq.cbs[i].out_offset;
-    work += k;
-    max_ckpt = std::max(max_ckpt, d.window / kSub + 1);
-    for (int w = 0; w < d.nwin; ++w) wincb.push_back(static_cast<int32_t>(i));
+    l.steps += k;
+    l.max_window = std::max(l.max_window, d.window);
+    l.max_windows = std::max(l.max_windows, d.nwin);
   }
-  const int n_win = static_cast<int>(wincb.size());
-  // Checkpoints live in a global scratch slot per window: 8 B of traffic per output step, and
-  // leaving shared memory unused gives the L1 cache the whole 256 KB for the input streams.
-  const size_t ckpt_bytes = static_cast<size_t>(kThreads) * max_ckpt * 2 * sizeof(float4);
-  const bool global_ckpt = rq.smem_checkpoints ? ckpt_bytes > static_cast<size_t>(smem_optin_)
-                                               : true;
 
-  // ---- device buffers ----
-  DevCb* dcbs = grow<DevCb>(d_cbs_, n);
-  int32_t* dwin = grow<int32_t>(d_wincb_, n_win);
-  float* sysi = grow<float>(d_sysi_, work);
-  float* e1i = grow<float>(d_e1i_, work);
-  float* e2 = grow<float>(d_e2_, work);
-  float* seeds = grow<float>(d_seed_, static_cast<size_t>(n_win) * 16 * 4);
-  uint8_t* done = grow<uint8_t>(d_done_, n);
-  uint32_t* iters = (rq.device_memory && rq.iterations_used) ? rq.iterations_used
-                                                              : grow<uint32_t>(d_iters_, n);
-  uint8_t* crc = (rq.device_memory && rq.crc_ok) ? rq.crc_ok : grow<uint8_t>(d_crc_, n);
-  const float* llr = rq.llr;
-  float* post = rq.posterior;
+  Io io;
+  io.iters = (rq.device_memory && rq.iterations_used) ? rq.iterations_used : grow<uint32_t>(d_iters_, n);
+  io.crc = (rq.device_memory && rq.crc_ok) ? rq.crc_ok : grow<uint8_t>(d_crc_, n);
+  io.llr = rq.llr;
+  io.post = rq.posterior;
   if (!rq.device_memory) {
     float* dl = grow<float>(d_llr_, rq.llr_len);
     check(cudaMemcpyAsync(dl, rq.llr, rq.llr_len * sizeof(float), cudaMemcpyHostToDevice, st),
           "copy LLRs in");
-    llr = dl;
-    post = grow<float>(d_post_, rq.post_len);
+    io.llr = dl;
+    io.post = grow<float>(d_post_, rq.post_len);
     // positions outside every block's range come back as 0
-    check(cudaMemsetAsync(post, 0, rq.post_len * sizeof(float), st), "zero posterior");
+    check(cudaMemsetAsync(io.post, 0, rq.post_len * sizeof(float), st), "zero posterior");
   }
-  float4* ckpt = nullptr;
-  if (global_ckpt) ckpt = grow<float4>(d_ckpt_, ckpt_slab(n_win, 2 * static_cast<size_t>(max_ckpt)));
+  pack_tasks(rq, l);
+  if (l.resident)
+    run_resident(rq, l, io, st, tape);
+  else
+    run_sweeps(rq, l, io, st, tape);
+  if (!rq.device_memory) {
+    check(cudaMemcpyAsync(rq.posterior, io.post, rq.post_len * sizeof(float), cudaMemcpyDeviceToHost, st),
+          "copy posterior out");
+    if (rq.crc_ok) check(cudaMemcpyAsync(rq.crc_ok, io.crc, n, cudaMemcpyDeviceToHost, st), "copy crc out");
+    if (rq.iterations_used)
+      check(cudaMemcpyAsync(rq.iterations_used, io.iters, n * 4, cudaMemcpyDeviceToHost, st),
+            "copy iters out");
+  }
+  mark_done(st);
+  if (!rq.device_memory) {
+    check(cudaStreamSynchronize(st), "sync");
+    if (rq.persistent) take_error();
+  }
+}
+
+// Packs the blocks into tasks for the block-resident kernel: largest first, whole blocks, one
+// thread per window, X within the shared memory of a CTA.  Leaves l.resident false when the
+// launch-per-half-iteration kernels are the better (or only) way.
+void Decoder::pack_tasks(const DecodeRequest& rq, Layout& l) const {
+  const size_t n = l.cbs.size();
+  if (rq.max_iterations > static_cast<uint32_t>(kMaxIterations) || l.max_windows > kResMaxThreads) return;
+  // threads per CTA: one warp when every block fits in it; else the multiple of 32 up to 128 that
+  // whole blocks of the largest window count fill best (48 windows of K = 6144 at 128 steps: two
+  // blocks in 96), unless the batch is too small to give every SM a CTA of several blocks
+  l.threads = l.max_windows > 128 ? 256 : (l.max_windows + 31) / 32 * 32;
+  if (l.max_windows > 32 && n > 2 * static_cast<size_t>(sm_count_)) {
+    double best = 0.0;
+    for (int t = l.threads; t <= 128; t += 32) {
+      const double use = static_cast<double>(t / l.max_windows * l.max_windows) / t;
+      if (use > best + 0.05) {
+        best = use;
+        l.threads = t;
+      }
+    }
+  }
+  size_t cap = res_x_bytes(32, 192) * static_cast<size_t>(l.threads / 32);  // 7 warps' worth per SM
+  for (const DevCb& d : l.cbs) cap = std::max(cap, res_x_bytes(d.nwin, d.window));
+  cap = std::min(cap, static_cast<size_t>(kResMaxX));
+  // counting sort by block size, largest first
+  std::vector<int32_t> start(kQppCount + 1, 0), order(n);
+  for (const DevCb& d : l.cbs) ++start[kQppCount - 1 - qpp_index(d.k) + 1];
+  for (int i = 0; i < kQppCount; ++i) start[i + 1] += start[i];
+  for (size_t i = 0; i < n; ++i) order[start[kQppCount - 1 - qpp_index(l.cbs[i].k)]++] = static_cast<int32_t>(i);
+  l.res.resize(n);
+  l.task_first.clear();
+  int lanes = 0, rows = 0;
+  size_t x = 0;
+  for (size_t j = 0; j < n; ++j) {
+    const DevCb& d = l.cbs[order[j]];
+    const int rows_with = std::max(rows, d.window);
+    if (j == 0 || lanes + d.nwin > l.threads || res_x_bytes(lanes + d.nwin, rows_with) > cap) {
+      if (res_x_bytes(d.nwin, d.window) > cap) return;  // does not fit at all
+      l.task_first.push_back(static_cast<int32_t>(j));
+      lanes = 0;
+      rows = 0;
+    }
+    rows = std::max(rows, d.window);
+    l.res[j] = ResCb{d.k, d.filler, d.tab, lanes, d.nwin, d.window, order[j], 0, d.llr, d.out};
+    lanes += d.nwin;
+    x = std::max(x, res_x_bytes(lanes, rows));
+  }
+  l.task_first.push_back(static_cast<int32_t>(n));
+  l.smem = x + res_head_bytes(l.threads);
+  const size_t tasks = l.task_first.size() - 1;
+  // windows above 1024 steps leave an SM fewer than 2 warps of lanes (X takes 4 bytes per step):
+  // the launch-per-half-iteration kernels run more windows at once, unless the whole batch is one
+  // wave anyway
+  const size_t per_sm = std::max<size_t>(1, static_cast<size_t>(228 * 1024) / (l.smem + 1024));
+  l.resident = l.max_window <= 1024 || tasks <= per_sm * sm_count_;
+}
+
+void Decoder::run_resident(const DecodeRequest& rq, const Layout& l, const Io& io, void* stream, const Tape* tape) {
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const size_t n = l.res.size();
+  const int tasks = static_cast<int>(l.task_first.size()) - 1;
+  const ResKernel f = res_kernel(rq.std3gpp, l.threads);
+  int per_sm = 0;
+  check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, l.threads, l.smem), "occupancy");
+  const int grid = std::min(tasks, sm_count_ * std::max(per_sm, 1));
+
+  ResArgs a{};
+  a.rows8 = l.max_window / 8;
+  a.slot = res_slot_planes(a.rows8) * l.threads;
+  a.scratch = grow<float4>(d_ckpt_, static_cast<size_t>(a.slot) * grid);
+  // descriptors: the blocks, the extrinsic scales, the tasks
+  const size_t at_scales = n * sizeof(ResCb), n_scales = 2 * static_cast<size_t>(rq.max_iterations);
+  const size_t at_tasks = at_scales + n_scales * sizeof(float);
+  std::vector<unsigned char> desc(at_tasks + l.task_first.size() * sizeof(int32_t));
+  std::memcpy(desc.data(), l.res.data(), n * sizeof(ResCb));
+  float* scales = reinterpret_cast<float*>(desc.data() + at_scales);
+  for (size_t i = 0; i < n_scales; ++i) scales[i] = rq.scales ? rq.scales[i] : 1.0f;
+  std::memcpy(desc.data() + at_tasks, l.task_first.data(), l.task_first.size() * sizeof(int32_t));
+  unsigned char* dd = grow<unsigned char>(d_rescbs_, desc.size());
+  upload(dd, desc.data(), desc.size(), st);
+  int* queue = grow<int>(d_queue_, 2);
+  const bool stall = rq.persistent && stall_task_ >= 0;
+  if (tasks > grid || stall) check(cudaMemsetAsync(queue, 0, 2 * sizeof(int), st), "zero queue");
+  a.cbs = reinterpret_cast<const ResCb*>(dd);
+  a.scale = reinterpret_cast<const float*>(dd + at_scales);
+  a.task_first = reinterpret_cast<const int32_t*>(dd + at_tasks);
+  a.n_tasks = tasks;
+  a.queue = queue;
+  a.never = queue + 1;
+  a.error = static_cast<int*>(d_err_.ptr);
+  a.stall_task = stall ? stall_task_ : -1;
+  a.llr = io.llr;
+  a.post = io.post;
+  a.perm = perm_table();
+  a.xpow = static_cast<const uint32_t*>(rq.std3gpp ? d_xpow_std_.ptr : d_xpow_.ptr);
+  a.guard = l.guard;
+  a.max_iterations = static_cast<int>(rq.max_iterations);
+  a.early_stop = rq.early_stop ? 1 : 0;
+  if (tape != nullptr) a.tape = *tape;
+  a.crc_ok = io.crc;
+  a.iters = io.iters;
+  record_start(st);
+  f<<<grid, l.threads, l.smem, st>>>(a);
+  check(cudaGetLastError(), "resident decoder launch");
+  record_stop(st, static_cast<uint64_t>(l.steps) * 2 * rq.max_iterations);
+  timing_.launches += 1;
+}
+
+namespace {
+// one SISO launch: kind 0 upper, 1 lower, 2 lower + posterior
+template <bool STD, bool TAPE>
+void launch_siso(int kind, int blocks, cudaStream_t st, const DevCb* dcbs, const int32_t* dwin,
+                 int n_win, const SisoIo& io, const uint8_t* dn, float4* ckpt) {
+  if (kind == 0) siso_plain_kernel<kSub, 0, STD, TAPE><<<blocks, kThreads, 0, st>>>(dcbs, dwin, n_win, io, dn, ckpt);
+  else if (kind == 1) siso_plain_kernel<kSub, 1, STD, TAPE><<<blocks, kThreads, 0, st>>>(dcbs, dwin, n_win, io, dn, ckpt);
+  else siso_plain_kernel<kSub, 2, STD, TAPE><<<blocks, kThreads, 0, st>>>(dcbs, dwin, n_win, io, dn, ckpt);
+}
+}  // namespace
+
+void Decoder::run_sweeps(const DecodeRequest& rq, const Layout& l, const Io& io, void* stream, const Tape* tape) {
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const size_t n = l.cbs.size();
+  std::vector<DevCb> cbs = l.cbs;
+  std::vector<int32_t> wincb;
+  for (size_t i = 0; i < n; ++i) {
+    cbs[i].win0 = static_cast<int32_t>(wincb.size());
+    for (int w = 0; w < cbs[i].nwin; ++w) wincb.push_back(static_cast<int32_t>(i));
+  }
+  const int n_win = static_cast<int>(wincb.size());
+  const int max_ckpt = l.max_window / kSub + 1;
+
+  // ---- device buffers (checkpoints in a global scratch slot per window) ----
+  DevCb* dcbs = grow<DevCb>(d_cbs_, n);
+  int32_t* dwin = grow<int32_t>(d_wincb_, n_win);
+  float* sysi = grow<float>(d_sysi_, l.steps);
+  float* e1i = grow<float>(d_e1i_, l.steps);
+  float* e2 = grow<float>(d_e2_, l.steps);
+  float* seeds = grow<float>(d_seed_, static_cast<size_t>(n_win) * 16 * 4);
+  uint8_t* done = grow<uint8_t>(d_done_, n);
+  float4* ckpt = grow<float4>(d_ckpt_, ckpt_slab(n_win, 2 * static_cast<size_t>(max_ckpt)));
 
   upload(dcbs, cbs.data(), n * sizeof(DevCb), st);
   upload(dwin, wincb.data(), n_win * sizeof(int32_t), st);
   check(cudaMemsetAsync(seeds, 0, static_cast<size_t>(n_win) * 16 * 4 * sizeof(float), st), "zero seeds");
   init_flags_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, st>>>(
-      static_cast<int>(n), done, iters, rq.max_iterations);
+      static_cast<int>(n), done, io.iters, rq.max_iterations);
   check(cudaGetLastError(), "init launch");
 
-  const uint16_t* dperm = static_cast<const uint16_t*>(d_perm_.ptr);
-  const uint16_t* dinv = static_cast<const uint16_t*>(d_inv_.ptr);
+  const uint16_t* dperm = perm_table();
+  const uint16_t* dinv = inv_table();
   timing_.launches += 3;  // init, setup, finish
-  launch_setup(dcbs, static_cast<int>(n), llr, dperm, sysi, e2, st);
+  launch_setup(dcbs, static_cast<int>(n), io.llr, dperm, sysi, e2, st);
   check(cudaGetLastError(), "setup launch");
 
   const int blocks = (n_win + kThreads - 1) / kThreads;
-  const size_t smem = global_ckpt ? 0 : ckpt_bytes;
   const size_t seed_slab = static_cast<size_t>(n_win) * 16;
   float* seed_up[2] = {seeds, seeds + seed_slab};
   float* seed_lo[2] = {seeds + 2 * seed_slab, seeds + 3 * seed_slab};
   for (uint32_t it = 0; it < rq.max_iterations; ++it) {
     const float s_up = rq.scales ? rq.scales[2 * it] : 1.0f;
     const float s_lo = rq.scales ? rq.scales[2 * it + 1] : 1.0f;
-    SisoIo up{llr, sysi, e2, e1i, nullptr, dperm, dinv, seed_up[it & 1], seed_up[(it + 1) & 1],
-              s_up, guard};
-    SisoIo lo{llr, sysi, e1i, e2, post, dperm, dinv, seed_lo[it & 1], seed_lo[(it + 1) & 1],
-              s_lo, guard};
+    SisoIo up{io.llr, sysi, e2, e1i, nullptr, dperm, dinv, seed_up[it & 1], seed_up[(it + 1) & 1],
+              s_up, l.guard};
+    SisoIo lo{io.llr, sysi, e1i, e2, io.post, dperm, dinv, seed_lo[it & 1], seed_lo[(it + 1) & 1],
+              s_lo, l.guard};
     const uint8_t* dn = rq.early_stop ? done : nullptr;
     // the posterior is needed after the last iteration and, with early stop, after each one
     const bool post_now = rq.early_stop || it + 1 == rq.max_iterations;
     for (int half = 0; half < 2; ++half) {
-      const SisoIo& io = half ? lo : up;
+      SisoIo sio = half ? lo : up;
+      if (tape != nullptr) {
+        const int j = 2 * it + half;
+        sio.tape = tape->s + j * tape->stride;
+        sio.seed_in = tape->seeds + j * tape->slab;
+        sio.seed_out = tape->seeds + (j + 2) * tape->slab;
+      }
       const int kind = half == 0 ? 0 : (post_now ? 2 : 1);
       record_start(st);
-      if (rq.std3gpp)
-        launch_plain<true>(kind, global_ckpt, blocks, smem, st, dcbs, dwin, n_win, io, dn, ckpt, max_ckpt);
-      else
-        launch_plain<false>(kind, global_ckpt, blocks, smem, st, dcbs, dwin, n_win, io, dn, ckpt, max_ckpt);
+      const auto launch = rq.std3gpp ? (tape ? launch_siso<true, true> : launch_siso<true, false>)
+                                     : (tape ? launch_siso<false, true> : launch_siso<false, false>);
+      launch(kind, blocks, st, dcbs, dwin, n_win, sio, dn, ckpt);
       check(cudaGetLastError(), "SISO launch");
-      record_stop(st, static_cast<uint64_t>(work));
+      record_stop(st, static_cast<uint64_t>(l.steps));
       timing_.launches += 1;
     }
     if (rq.early_stop) {
       crc_stop_kernel<<<static_cast<unsigned>((n * 32 + 255) / 256), 256, 0, st>>>(
-          dcbs, static_cast<int>(n), post,
-          static_cast<const uint32_t*>(rq.std3gpp ? d_xpow_std_.ptr : d_xpow_.ptr), done, iters,
+          dcbs, static_cast<int>(n), io.post,
+          static_cast<const uint32_t*>(rq.std3gpp ? d_xpow_std_.ptr : d_xpow_.ptr), done, io.iters,
           static_cast<int>(it));
       check(cudaGetLastError(), "CRC launch");
       timing_.launches += 1;
     }
   }
-  finish_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, st>>>(static_cast<int>(n), done, crc,
+  finish_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, st>>>(static_cast<int>(n), done, io.crc,
                                                                          rq.early_stop ? 1 : 0);
   check(cudaGetLastError(), "finish launch");
-  if (!rq.device_memory) {
-    check(cudaMemcpyAsync(rq.posterior, post, rq.post_len * sizeof(float), cudaMemcpyDeviceToHost, st),
-          "copy posterior out");
-    if (rq.crc_ok) check(cudaMemcpyAsync(rq.crc_ok, crc, n, cudaMemcpyDeviceToHost, st), "copy crc out");
-    if (rq.iterations_used)
-      check(cudaMemcpyAsync(rq.iterations_used, iters, n * 4, cudaMemcpyDeviceToHost, st), "copy iters out");
-  }
-  mark_done(st);
-  if (!rq.device_memory) check(cudaStreamSynchronize(st), "sync");
 }
 
 // ------------------------------------------------------------------------------------------
@@ -735,7 +908,7 @@ void Decoder::decode_host_async(const DecodeRequest& rq) {
   // the decode follows the previous call's decode (another worker); the copy-in above does not
   if (last_compute_)
     check(cudaStreamWaitEvent(ws, static_cast<cudaEvent_t>(last_compute_), 0), "cudaStreamWaitEvent");
-  if (r.persistent) w.decode_persistent(r); else w.decode_plain(r);
+  w.decode_now(r);
   check(cudaEventRecord(static_cast<cudaEvent_t>(w.compute_event()), ws), "cudaEventRecord");
   last_compute_ = w.compute_done_;
   check(cudaMemcpyAsync(rq.posterior, dp, rq.post_len * sizeof(float), cudaMemcpyDeviceToHost, ws),
@@ -747,177 +920,6 @@ void Decoder::decode_host_async(const DecodeRequest& rq) {
                           cudaMemcpyDeviceToHost, ws), "copy iters out");
   w.mark_done(ws);
   timing_.launches += w.timing_.launches - launches_before;
-}
-
-// ------------------------------------------------------------------------------------------
-// Persistent schedule: warp tasks of whole code blocks, one launch for all iterations.
-// ------------------------------------------------------------------------------------------
-void Decoder::decode_persistent(const DecodeRequest& rq) {
-  check(cudaSetDevice(device_), "cudaSetDevice");
-  cudaStream_t st = static_cast<cudaStream_t>(rq.device_memory ? rq.stream
-                                                               : (rq.stream ? rq.stream : stream_));
-  const size_t n = rq.n_cb;
-  if (n == 0) return;
-  if (reinterpret_cast<uintptr_t>(rq.llr) % 16 != 0)
-    throw InvalidArgument("the LLR buffer must be 16-byte aligned");
-  order_after_previous(st);
-  if (rq.max_iterations > static_cast<uint32_t>(kMaxIterations))
-    throw InvalidArgument("max_iterations above 64");
-  const int guard = rq.guard < 0 ? kDefaultGuard : rq.guard;
-  if (guard % kGroup != 0) throw InvalidArgument("guard must be a multiple of 8");
-  const int target = rq.window > 0 ? rq.window : kPersistWindow;
-
-  // ---- per block: at most 32 windows of >= `target` steps (a multiple of 8, >= guard) ----
-  std::vector<DevCb> cbs(n);
-  int64_t work = 0;
-  int max_ckpt = 0;
-  for (size_t i = 0; i < n; ++i) {
-    const int32_t k = rq.cbs[i].k;
-    const int qi = qpp_index(k);
-    if (qi < 0) throw OutOfRange("unsupported QPP block size");
-    if (rq.cbs[i].filler < 0 || rq.cbs[i].filler >= k) throw InvalidArgument("invalid filler count");
-    if (rq.cbs[i].llr_offset < 0 || rq.cbs[i].llr_offset % 4 != 0 ||
-        static_cast<size_t>(rq.cbs[i].llr_offset) + 3 * static_cast<size_t>(k + 4) > rq.llr_len)
-      throw InvalidArgument("invalid LLR offset (must be a multiple of 4 and in range)");
-    if (rq.cbs[i].out_offset < 0 ||
-        static_cast<size_t>(rq.cbs[i].out_offset) + static_cast<size_t>(k) > rq.post_len)
-      throw InvalidArgument("invalid posterior offset");
-    DevCb& d = cbs[i];
-    d.k = k;
-    d.filler = rq.cbs[i].filler;
-    d.tab = tab_offset_[qi];
-    int nwin = std::max(1, std::min(32, k / std::max(target, 8)));
-    int wlen = ((k + nwin - 1) / nwin + kGroup - 1) / kGroup * kGroup;
-    if (nwin > 1 && wlen < guard) {  // windows may not be shorter than the guard
-      nwin = std::max(1, k / guard);
-      wlen = ((k + nwin - 1) / nwin + kGroup - 1) / kGroup * kGroup;
-    }
-    d.window = std::min<int32_t>(wlen, k);
-    d.nwin = (k + d.window - 1) / d.window;
-    d.llr = rq.cbs[i].llr_offset;
-    d.work = work;
-    d.out = rq.cbs[i].out_offset;
-    work += k;
-    max_ckpt = std::max(max_ckpt, d.window / kSub + 1);
-  }
-  // ---- tasks: blocks sorted by size, largest first, packed first-fit into 32 lanes ----
-  std::vector<int32_t> order(n);
-  for (size_t i = 0; i < n; ++i) order[i] = static_cast<int32_t>(i);
-  std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) {
-    return cbs[a].nwin != cbs[b].nwin ? cbs[a].nwin > cbs[b].nwin : cbs[a].k > cbs[b].k;
-  });
-  std::vector<int32_t> wincb, tasks;
-  int lanes_used = 32;
-  for (const int32_t i : order) {
-    DevCb& d = cbs[i];
-    if (lanes_used + d.nwin > 32) {  // open a new task
-      tasks.insert(tasks.end(), 32, -1);
-      lanes_used = 0;
-    }
-    d.win0 = static_cast<int32_t>(wincb.size());
-    for (int w = 0; w < d.nwin; ++w) {
-      tasks[tasks.size() - 32 + lanes_used + w] = static_cast<int32_t>(wincb.size());
-      wincb.push_back(i);
-    }
-    lanes_used += d.nwin;
-  }
-  const int n_tasks = static_cast<int>(tasks.size() / 32);
-  const int n_win = static_cast<int>(wincb.size());
-
-  // ---- device buffers ----
-  DevCb* dcbs = grow<DevCb>(d_cbs_, n);
-  int32_t* dwin = grow<int32_t>(d_wincb_, n_win);
-  int32_t* dtasks = grow<int32_t>(d_tasks_, tasks.size());
-  int* dqueue = grow<int>(d_queue_, 2 + static_cast<size_t>(n_tasks));  // queue, error, progress
-  float* sysi = grow<float>(d_sysi_, work);
-  float* e1i = grow<float>(d_e1i_, work);
-  float* e2 = grow<float>(d_e2_, work);
-  float* seeds = grow<float>(d_seed_, static_cast<size_t>(n_win) * 16 * 4);
-  float4* ckpt = grow<float4>(d_ckpt_, ckpt_slab(n_win, 2 * static_cast<size_t>(max_ckpt)));
-  uint8_t* done = grow<uint8_t>(d_done_, n);
-  uint32_t* iters = (rq.device_memory && rq.iterations_used) ? rq.iterations_used
-                                                              : grow<uint32_t>(d_iters_, n);
-  uint8_t* crc = (rq.device_memory && rq.crc_ok) ? rq.crc_ok : grow<uint8_t>(d_crc_, n);
-  const float* llr = rq.llr;
-  float* post = rq.posterior;
-  if (!rq.device_memory) {
-    float* dl = grow<float>(d_llr_, rq.llr_len);
-    check(cudaMemcpyAsync(dl, rq.llr, rq.llr_len * sizeof(float), cudaMemcpyHostToDevice, st),
-          "copy LLRs in");
-    llr = dl;
-    post = grow<float>(d_post_, rq.post_len);
-    check(cudaMemsetAsync(post, 0, rq.post_len * sizeof(float), st), "zero posterior");
-  }
-  upload(dcbs, cbs.data(), n * sizeof(DevCb), st);
-  upload(dwin, wincb.data(), n_win * sizeof(int32_t), st);
-  upload(dtasks, tasks.data(), tasks.size() * sizeof(int32_t), st);
-  check(cudaMemsetAsync(dqueue, 0, (2 + static_cast<size_t>(n_tasks)) * sizeof(int), st),
-        "zero queue");
-  check(cudaMemsetAsync(seeds, 0, static_cast<size_t>(n_win) * 16 * 4 * sizeof(float), st),
-        "zero seeds");
-  init_flags_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, st>>>(
-      static_cast<int>(n), done, iters, rq.max_iterations);
-  launch_setup(dcbs, static_cast<int>(n), llr, static_cast<const uint16_t*>(d_perm_.ptr), sysi,
-               e2, st);
-  check(cudaGetLastError(), "set-up launch");
-
-  PersistArgs a{};
-  a.cbs = dcbs;
-  a.win_cb = dwin;
-  a.tasks = dtasks;
-  a.n_tasks = n_tasks;
-  a.queue = dqueue;
-  a.error = static_cast<int*>(d_err_.ptr);
-  a.stall_task = stall_task_;
-  a.progress = dqueue + 2;
-  a.llr = llr;
-  a.sys_i = sysi;
-  a.e1i = e1i;
-  a.e2 = e2;
-  a.post = post;
-  a.perm = static_cast<const uint16_t*>(d_perm_.ptr);
-  a.inv = static_cast<const uint16_t*>(d_inv_.ptr);
-  const size_t slab = static_cast<size_t>(n_win) * 16;
-  a.seed_up[0] = seeds;
-  a.seed_up[1] = seeds + slab;
-  a.seed_lo[0] = seeds + 2 * slab;
-  a.seed_lo[1] = seeds + 3 * slab;
-  a.ckpt = ckpt;
-  a.ckpt_per_window = max_ckpt;
-  a.n_windows = n_win;
-  a.guard = guard;
-  a.max_iterations = static_cast<int>(rq.max_iterations);
-  a.early_stop = rq.early_stop ? 1 : 0;
-  a.done = done;
-  a.iters = iters;
-  a.xpow = static_cast<const uint32_t*>(rq.std3gpp ? d_xpow_std_.ptr : d_xpow_.ptr);
-  for (int i = 0; i < 2 * kMaxIterations; ++i)
-    a.scale[i] = (rq.scales && i < 2 * static_cast<int>(rq.max_iterations)) ? rq.scales[i] : 1.0f;
-  const int grid = std::max(1, sm_count_ * std::max(persist_blocks_per_sm_, 1));
-  record_start(st);
-  if (rq.std3gpp)
-    persistent_kernel<true><<<grid, kPersistThreads, 0, st>>>(a);
-  else
-    persistent_kernel<false><<<grid, kPersistThreads, 0, st>>>(a);
-  check(cudaGetLastError(), "persistent launch");
-  record_stop(st, static_cast<uint64_t>(work) * 2 * rq.max_iterations);
-  finish_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, st>>>(static_cast<int>(n), done,
-                                                                         crc, rq.early_stop ? 1 : 0);
-  check(cudaGetLastError(), "finish launch");
-  timing_.launches += 4;
-  if (!rq.device_memory) {
-    check(cudaMemcpyAsync(rq.posterior, post, rq.post_len * sizeof(float), cudaMemcpyDeviceToHost, st),
-          "copy posterior out");
-    if (rq.crc_ok) check(cudaMemcpyAsync(rq.crc_ok, crc, n, cudaMemcpyDeviceToHost, st), "copy crc out");
-    if (rq.iterations_used)
-      check(cudaMemcpyAsync(rq.iterations_used, iters, n * 4, cudaMemcpyDeviceToHost, st),
-            "copy iters out");
-    mark_done(st);
-    check(cudaStreamSynchronize(st), "sync");
-    take_error();
-  } else {
-    mark_done(st);
-  }
 }
 
 }  // namespace tcb

@@ -38,6 +38,8 @@ constexpr int kGroup = 8;            // load granularity: windows and guards are
 constexpr int kDefaultWindow = 128;  // window length (steps)
 constexpr int kDefaultGuard = 96;    // warm-up steps on each side of a window
 constexpr int kPersistWindow = 192;  // target window of the persistent schedule (<= 32 per block)
+constexpr int kMaxIterations = 64;   // of the persistent schedule and the block-resident kernel
+constexpr int kXpowSize = 6144 + 32;  // x^j mod g_CRC24B table (a window's 24-bit part times x^j)
 constexpr size_t kAsyncWorkers = 3;  // TC_MEM_HOST_ASYNC workspaces: call i+2's copy-in needs no wait for call i
 
 struct CodeBlockDesc {
@@ -45,6 +47,19 @@ struct CodeBlockDesc {
   int32_t filler;
   int64_t llr_offset;  // floats; [d0|d1|d2], 3*(K+4) floats, multiple of 4
   int64_t out_offset;  // floats; K posterior LLRs
+};
+
+// Where a taped forward pass leaves what each half-iteration j reads: log2(e) (Ls + La) in the SISO's
+// order at s + j * stride + DevCb::work, the seeds (alpha, beta) of window DevCb::win0 + w at
+// seeds + j * slab + 16 (win0 + w).  Room for 2 slabs more: a launch per half-iteration writes the
+// seeds of j + 2; the first two are zero.
+struct DevCb;
+struct Tape {
+  const DevCb* cbs = nullptr;  // device; work and win0 of each block of the request, in its order
+  float* s = nullptr;
+  int64_t stride = 0;
+  float* seeds = nullptr;
+  int64_t slab = 0;
 };
 
 struct DecodeRequest {
@@ -62,8 +77,7 @@ struct DecodeRequest {
   int guard = -1;   // <0: default
   bool device_memory = false;  // llr/posterior/crc_ok/iterations_used are device pointers
   bool host_async = false;     // host pointers; enqueue copies + decode and return (see sync())
-  bool smem_checkpoints = false;  // alpha checkpoints in shared memory instead of global scratch
-  bool persistent = false;  // persistent warp-task schedule instead of per-half-iteration launches
+  bool persistent = false;  // window layout: at most 32 windows per block instead of a fixed length
   bool graph = false;       // device memory: capture the launch sequence once, replay it after
   bool auto_schedule = false;  // take schedule and window from the autotuning table
   const float* scales = nullptr;  // host; 2 per iteration (upper, lower); null = all 1
@@ -133,6 +147,9 @@ class Decoder {
   Decoder(const Decoder&) = delete;
   Decoder& operator=(const Decoder&) = delete;
 
+  // A device-memory decode that also records the tape of its half-iterations (the differentiable
+  // decoder's forward pass); returns the kernels launched.
+  uint64_t decode_taped(const DecodeRequest& rq, const Tape& tape);
   void decode(const DecodeRequest& rq);  // plain or persistent schedule
   int device() const { return device_; }
   void set_timing(bool on);
@@ -177,9 +194,16 @@ class Decoder {
   int32_t table_offset(int32_t k) const;
 
  private:
-  int pick_window(int32_t k, int32_t requested) const;
-  void decode_persistent(const DecodeRequest& rq);
-  void decode_plain(const DecodeRequest& rq);
+  // One decode: checks the request, cuts the blocks into windows (the two schedules differ in
+  // the layout only) and runs the block-resident kernel, or, for layouts it cannot hold, one
+  // launch per half-iteration.
+  void decode_now(const DecodeRequest& rq, const Tape* tape = nullptr);
+  struct Layout;  // windows of a request and their packing into tasks (decoder.cu)
+  struct Io;      // device buffers of one call
+  void check_request(const DecodeRequest& rq) const;
+  void pack_tasks(const DecodeRequest& rq, Layout& l) const;
+  void run_resident(const DecodeRequest& rq, const Layout& l, const Io& io, void* stream, const Tape* tape);
+  void run_sweeps(const DecodeRequest& rq, const Layout& l, const Io& io, void* stream, const Tape* tape);
   // Asynchronous host-memory calls rotate over kAsyncWorkers worker decoders, each with its own
   // device buffers and stream: a call enqueues copy-in, decode and copy-out on the next worker
   // and returns, so that its copies run while the previous calls decode.  sync() waits for them.
@@ -245,13 +269,12 @@ class Decoder {
   std::vector<int32_t> tab_offset_;
   DeviceBuffer d_perm_, d_inv_, d_xpow_, d_xpow_std_;  // x^j mod g_CRC24B: reference, TS 36.212
   DeviceBuffer d_cbs_, d_wincb_, d_llr_, d_sysi_, d_e1i_, d_e2_, d_post_, d_seed_,
-      d_done_, d_iters_, d_crc_, d_ckpt_, d_tasks_, d_queue_;
+      d_done_, d_iters_, d_crc_, d_ckpt_, d_queue_, d_rescbs_;
   DeviceBuffer d_rmgroup_, d_gen_, d_gentab_, d_genenc_, d_genrm_, d_xpow_a_std_;
   DeviceBuffer d_tbcb_, d_synpart_;
   DeviceBuffer d_rm_, d_e_llr_, d_d012_, d_tbpost_, d_tbbits_, d_tbok_, d_cbok_, d_tbiters_, d_tb_,
       d_xpow_a_;
-  int persist_blocks_per_sm_ = 0;
-  DeviceBuffer d_err_;          // sticky: set by a persistent-schedule wait that gave up
+  DeviceBuffer d_err_;          // sticky: set by a device-side wait that gave up
   int stall_task_ = -1;
   void* last_event_ = nullptr;  // completion of the previous decode (orders workspace reuse)
   // Host-async calls: the decode of each call waits for the previous call's decode (on another

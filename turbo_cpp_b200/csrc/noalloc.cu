@@ -218,14 +218,11 @@ void decode_noalloc(const DecodeRequest& rq, size_t* bytes_needed) {
                     seed_lo[(it + 1) & 1], s_lo, guard};
     const uint8_t* dn = rq.early_stop ? done : nullptr;
     const bool post_now = rq.early_stop || it + 1 == rq.max_iterations;
-    siso_plain_kernel<kSub, 0, true><<<blocks, kThreads, 0, st>>>(dcbs, dwin, n_win, up, dn, ckpt,
-                                                                  max_ckpt);
+    siso_plain_kernel<kSub, 0><<<blocks, kThreads, 0, st>>>(dcbs, dwin, n_win, up, dn, ckpt);
     if (post_now)
-      siso_plain_kernel<kSub, 2, true><<<blocks, kThreads, 0, st>>>(dcbs, dwin, n_win, lo, dn, ckpt,
-                                                                    max_ckpt);
+      siso_plain_kernel<kSub, 2><<<blocks, kThreads, 0, st>>>(dcbs, dwin, n_win, lo, dn, ckpt);
     else
-      siso_plain_kernel<kSub, 1, true><<<blocks, kThreads, 0, st>>>(dcbs, dwin, n_win, lo, dn, ckpt,
-                                                                    max_ckpt);
+      siso_plain_kernel<kSub, 1><<<blocks, kThreads, 0, st>>>(dcbs, dwin, n_win, lo, dn, ckpt);
     ok(cudaGetLastError(), "SISO launch");
     if (rq.early_stop) {
       crc_stop_kernel<<<static_cast<unsigned>((n * 32 + 255) / 256), 256, 0, st>>>(

@@ -1,0 +1,1189 @@
+// resident.cuh -- the block-resident decoder: one launch for all iterations, a CTA per task.
+//
+// A task is one or more whole code blocks, one thread per window, and a CTA keeps it from the
+// first half-iteration to the last: the LLR that every half-iteration reads (Ls + the other SISO's
+// extrinsic) stays in shared memory for the whole decode, in natural order, so neither SISO needs
+// an interleaved copy and no half-iteration waits for another CTA.  The streams that are only read
+// (parities, systematic) and the alpha checkpoints sit in a scratch slot per resident CTA, laid
+// out so that the lanes of a warp access consecutive words; the slots are reused from task to task
+// and stay in L2.
+//
+// Arithmetic: the state metrics are kept as probabilities (float32, scaled by powers of two), not
+// as logarithms.  A trellis step of the 8 states is 16 multiply-adds and two ex2 for the branch
+// weights, where the (m, s) form of trellis.cuh needs 8 ex2 and about 85 instructions; the
+// extrinsic is one lg2 of each of two 4-term sums.  What limits it is float's exponent range: a
+// probability below 2^-149 becomes 0.  Each step checks that what it computed cannot have lost
+// anything that matters (kLost below); a block that fails goes on in the (m, s) form (siso.cuh),
+// from there or from the start, in a second pass.  LLRs of ordinary channels stay inside the range (extrinsics of
+// about 120 to 170 bits, depending on the parities; eight iterations at 1/3 reach 90 bits at 1 dB, 143 at
+// 2.5 dB); blocks of rate 4/5 that fail their CRC may leave it, scaled-up LLRs do.
+//
+// The linear pass keeps all LLRs in base-2 units (natural LLR * log2(e)).
+//
+// What bounds it: the issue slots of the SMs (158 instructions per step of a half-iteration, warm-ups
+// included, 84 of them multiply-adds; the (m, s) form has about 450), at 2 warps per scheduler.  One warp
+// of 32 windows of 192 steps per CTA, because the shared memory of an SM holds X of 8 of them: 4096
+// blocks of K = 6144, 8 iterations: 2.83 ms with 8 CTAs per SM, 2.94 ms with 7 (rows of 33 words and a
+// ring of 4 stages), 8.5 ms with the (m, s) kernel that this one replaced.  One block of K = 6144 from
+// host memory: 0.44 ms (1.09 ms); 20000 mixed blocks with early stop: 6.8 ms (14.2 ms).
+#pragma once
+#include <cuda_runtime.h>
+
+#include <cstdint>
+
+#include "decoder.hpp"
+#include "siso.cuh"
+
+namespace tcb {
+namespace {
+
+constexpr int kResMaxThreads = 256;
+constexpr int kResMaxX = 65536 - 256;             // bytes of X: its offsets are 16 bits
+constexpr int kResMaxSmem = 227 * 1024;
+constexpr uint64_t kWaitLimitNs = 1000000000ull;  // of a device-side wait: one second
+
+// One code block as the kernel sees it; the blocks of a task are consecutive in the list.
+struct ResCb {
+  int32_t k, filler;
+  int32_t tab;     // offset of this K's permutation table
+  int32_t lane0;   // thread of the block's first window within its task
+  int32_t nwin, window;
+  int32_t idx;     // the caller's index of the block (flags, iteration counts)
+  int32_t pad;
+  int64_t llr;     // float offset of [d0|d1|d2]
+  int64_t out;     // float offset of the posterior
+};
+
+struct ResArgs {
+  const ResCb* cbs;
+  const int32_t* task_first;  // [n_tasks + 1]: first block of each task
+  int n_tasks;
+  int* queue;                 // next task beyond the grid (zero before the launch)
+  const int* never;           // testing hook: a word that stays 0
+  int* error;
+  int stall_task;             // testing hook (-1: off)
+  const float* llr;
+  float* post;
+  const uint16_t* perm;
+  const uint32_t* xpow;       // x^j mod g_CRC24B, kXpowSize entries, then b(x) x^24 mod g per byte b
+  float4* scratch;
+  int64_t slot;               // float4 per scratch slot (one slot per CTA of the grid)
+  int rows8;                  // longest window of the call / 8
+  int guard;
+  int max_iterations;
+  int early_stop;
+  uint8_t* crc_ok;
+  uint32_t* iters;
+  const float* scale;         // [2 * max_iterations]
+  Tape tape;                  // of a taped forward pass (tape.s null: none)
+};
+
+__device__ __forceinline__ int load_acquire(const int* p) {
+  int v;
+  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint64_t global_ns() {
+  uint64_t t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+
+// Scratch slot of a CTA of NT threads, in planes of NT float4 (rows8 = longest window / 8, one record
+// per 8 steps):
+//   upper SISO: rows8 records of parity 1 (2 planes), the shared-memory byte offsets of the 8
+//     positions (8 x uint16: 1), systematic (2)
+//   lower SISO: the same of parity 2 and the interleaved positions
+//   alpha checkpoints, one per 8 steps (the extrinsics of the 8 steps replace it): 2 rows8
+//   what the half-iteration read, for a second pass that takes over from there: 2 rows8
+//   (second pass: behind the extrinsics, checkpoints of the (m, s) form, one per 4 steps, and one
+//   more): 4 rows8 + 2
+//   seeds: 2 SISOs x 2 iteration parities x (alpha, beta) x 2 planes: 16
+//   beta at the block end (log values) of the upper and the lower SISO: 4
+//   the windows (k, window, nwin, lane0: 4 x uint16): 1
+// Both SISOs take their places in X from the record, so that they share one copy of the code (with a
+// copy each, the phases that the warps of an SM are in at a time overflow the instruction cache).
+__host__ __device__ inline int64_t res_slot_planes(int rows8) { return 16 * static_cast<int64_t>(rows8) + 23; }
+
+// Scaling and checks.  The branch weights of a step are below 2, so that the largest metric grows by at
+// most 3 per step; every 8 steps it is set to 2^top, as high as the block's largest parity weight
+// leaves room for in the products (res_top).  What falls below float's range is an absolute error of
+// 2^-150 in a metric: a path cut off there weighs at most 2^-150 2^(top + 13) of a mass of all paths (the
+// sum of alpha beta, the same throughout a group of 8 steps).  The smaller side of an extrinsic x has
+// 2^-|x| of the mass and must be 2^kKept times what was lost anywhere in the block (half an ulp of
+// an x of 64 or more), so that a block passes if
+//   log2(smallest mass) - max |x| >= top + 13 - 150 + kKept.
+// An input weight below 2^-126 is flushed; the paths lost with it weigh 2^-126 times their side of the
+// extrinsic x there, 2^(-126 - x) where x favours the other input.
+constexpr int kKept = 18;
+// A block within kNear of that keeps what its half-iterations read, so that the second pass can go on
+// there (a store more per step: 14 % of the time if all did); one that fails from further off starts again.
+constexpr float kNear = 40.0f;
+constexpr float kLost = 150.0f - 13.0f - kKept;
+constexpr float kMaxParity = 76.0f;  // larger ones go to the second pass at once
+constexpr int kTopMax = 60;
+// top of a block whose largest parity weight is 2^q: leaves the products of a step 18 bits of growth
+// below 2^126 (on ordinary channels alpha and beta grow by 4 or 5 each)
+__device__ __forceinline__ int res_top(float q) {
+  return min(kTopMax, static_cast<int>(0.5f * (108.0f - fminf(q, kMaxParity))));
+}
+
+// min(x, y), max(x, y, z), NaN if any is
+__device__ __forceinline__ float min_nan(float x, float y) {
+  float r;
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ float max3_nan(float x, float y, float z) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(x), "f"(y), "f"(z));
+  return r;
+}
+
+// Branch weights of one step from s = log2(e) (Ls + La) and b = 2^(log2(e) Lp): input 1 / input 0 and
+// parity 1 (parity 0: 1).  The input weights carry the power of two that keeps the likeliest branch
+// below 2.  (2^(log2(e) Lp) is in the record: a step needs one ex2 here, not two or three, and the
+// unit that computes it was busy for half of the time.)
+struct Weights {
+  float a1, a0, b;
+};
+__device__ __forceinline__ Weights weights(float s, float b) {
+  const float y = __int_as_float(0x7f000000 - (__float_as_int(fmaxf(b, 1.0f)) & 0x7f800000));
+  const float x = ex2(-fabsf(s)) * y;
+  return Weights{s < 0.0f ? x : y, s < 0.0f ? y : x, b};
+}
+
+// log2(x / y) of positive normal x, y (y < 2^126): the exponents' difference is exact and what is left
+// of the ratio is in [1, 2), so that the result is rounded once at its own size.  (lg2 of each side,
+// of the size of the scaled metrics, is 6 instructions shorter and 3 times further off.)
+__device__ __forceinline__ float log_ratio(float x, float y) {
+  const int d = (__float_as_int(x) - __float_as_int(y)) & 0xff800000;
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
+  const float e = __int_as_float((d >> 23) + 0x4b400000) - 12582912.0f;  // d 2^-23
+  return e + lg2(__int_as_float(__float_as_int(x) - d) * r);
+}
+
+// The scale 2^(top - exponent of the largest of m).
+__device__ __forceinline__ float rescale(const float (&m)[8], int top) {
+  const float x = max3(max3(m[0], m[1], m[2]), max3(m[3], m[4], m[5]), max3(m[6], m[7], 0x1p-60f));
+  return __int_as_float(((top + 254) << 23) - (__float_as_int(x) & 0x7f800000));
+}
+
+// Reference code: at[n] = sum over the two branches into n of alpha * parity weight; the input
+// weight is common to both (pred_input depends on n only) and is applied by alpha_scale.
+__device__ __forceinline__ void alpha_lin(const float (&al)[8], float b, float (&at)[8]) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float x = al[2 * j], y = al[2 * j + 1];
+    const float u = fmaf(b, y, x), v = fmaf(b, x, y);
+    at[j] = j < 2 ? u : v;
+    at[j + 4] = j < 2 ? v : u;
+  }
+}
+__device__ __forceinline__ void input_scale(const float (&at)[8], float a1, float a0, float (&al)[8]) {
+#pragma unroll
+  for (int n = 0; n < 8; ++n) al[n] = at[n] * (pred_input<false>(n, 0) ? a1 : a0);
+}
+// beta_t from beta_{t+1} times the input weights
+__device__ __forceinline__ void beta_lin(const float (&bh)[8], float b, float (&be)[8]) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float x = bh[j], y = bh[j + 4];
+    const float u = fmaf(b, y, x), v = fmaf(b, x, y);
+    be[2 * j] = j < 2 ? u : v;
+    be[2 * j + 1] = j < 2 ? v : u;
+  }
+}
+// The TS 36.212 code: both input and parity weights differ between the branches into a state.
+__device__ __forceinline__ void std_weights(const Weights& w, float (&g)[2][2]) {
+  g[0][0] = w.a0;
+  g[0][1] = w.a0 * w.b;
+  g[1][0] = w.a1;
+  g[1][1] = w.a1 * w.b;
+}
+__device__ __forceinline__ void alpha_std(const float (&al)[8], const float (&g)[2][2], float (&out)[8]) {
+#pragma unroll
+  for (int n = 0; n < 8; ++n) {
+    const int p0 = 2 * (n & 3);
+    out[n] = fmaf(al[p0], g[pred_input<true>(n, 0)][pred_parity(n, 0)],
+                  al[p0 + 1] * g[pred_input<true>(n, 1)][pred_parity(n, 1)]);
+  }
+}
+__device__ __forceinline__ void beta_std(const float (&be)[8], const float (&g)[2][2], float (&out)[8]) {
+#pragma unroll
+  for (int s = 0; s < 8; ++s)
+    out[s] = fmaf(be[next_state<true>(s, 0)], g[0][parity<true>(s, 0)],
+                  be[next_state<true>(s, 1)] * g[1][parity<true>(s, 1)]);
+}
+
+// One alpha step with weights w, one beta step with weights w scaled by r.
+template <bool STD>
+__device__ __forceinline__ void alpha_next(float (&al)[8], const Weights& w) {
+  float t[8];
+  if constexpr (STD) {
+    float g[2][2];
+    std_weights(w, g);
+    alpha_std(al, g, t);
+#pragma unroll
+    for (int n = 0; n < 8; ++n) al[n] = t[n];
+  } else {
+    alpha_lin(al, w.b, t);
+    input_scale(t, w.a1, w.a0, al);
+  }
+}
+template <bool STD>
+__device__ __forceinline__ void beta_next(float (&be)[8], Weights w, float r) {
+  w.a1 *= r;
+  w.a0 *= r;
+  float t[8];
+  if constexpr (STD) {
+    float g[2][2];
+    std_weights(w, g);
+    beta_std(be, g, t);
+#pragma unroll
+    for (int n = 0; n < 8; ++n) be[n] = t[n];
+  } else {
+    input_scale(be, w.a1, w.a0, t);
+    beta_lin(t, w.b, be);
+  }
+}
+
+// log2 metrics (largest 0) <-> scaled probabilities, down to float's smallest (ex2 and lg2 flush
+// what is below 2^-126)
+__device__ __forceinline__ void lin_from_log(const float (&v)[8], float (&m)[8], int top) {
+  const float x = static_cast<float>(top + 24) - max8(v);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) m[k] = 0x1p-24f * ex2(v[k] + x);
+}
+__device__ __forceinline__ void log_from_lin(const float (&m)[8], float (&v)[8]) {
+  float r[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) r[k] = fmaxf(lg2(0x1p24f * m[k]), kNegBig);
+  const float x = max8(r);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) v[k] = fmaxf(r[k] - x, kNegBig);
+}
+
+// The phases of a decode are functions of their own (not inlined: in one function their address
+// arithmetic is hoisted out of the iteration loops and spilled), so what they need is kept in shared
+// memory: the CTA's constants and, per thread, its window.
+// Words between the rows of X: the warp's windows in consecutive banks.  An odd number keeps the columns
+// (inputs and outputs) free of bank conflicts too; full warps do without, because 8 CTAs of 32
+// windows of 192 steps then fit in an SM.
+__host__ __device__ inline int res_pitch(int lanes) { return lanes % 32 == 0 ? lanes : lanes | 1; }
+struct ResCta {
+  char* slot;          // the CTA's scratch slot
+  int guard;
+  int rows8;
+  uint32_t xs4;        // bytes between the rows of X
+  int max_window;      // of the task
+  int next_task;
+  uint32_t crc_tab[16];  // b(x) x^24 mod g of the 4-bit b
+};
+// Dynamic shared memory of a CTA of NT threads: ResCta; a word per thread, used at the first thread of a
+// block (kWordPar); the ring; X.  Between two passes over the streams the ring is idle, and three words per
+// thread in it (kWordExt ..) pass a half-iteration's checks and the CRC between the block's threads.
+extern __shared__ __align__(16) char res_smem[];
+constexpr int kResHead = (sizeof(ResCta) + 15) / 16 * 16;
+// Streams of the slot come through a ring in shared memory (cp.async, each thread its own
+// entries), because the slots of all resident CTAs together are about as large as L2: a group of
+// 8 steps is requested several groups before its use, which covers a DRAM access without holding
+// registers.  Stage: entries of 16 bytes per thread, [entry][thread].
+constexpr int kStages = 2;
+constexpr int kEntries = 3;  // of a stage: 2 of parity, 1 of positions
+__host__ __device__ constexpr int res_ring_at(int nt) { return kResHead + 4 * nt; }
+__host__ __device__ constexpr int res_x_at(int nt) { return res_ring_at(nt) + 16 * kStages * kEntries * nt; }
+
+// What one thread knows of its window.
+struct ResWin {
+  int k, w, nwin, lo, len;   // block size, window, windows, first step, steps
+  int window, guard;
+  int tid, lane0;
+  int prev, next;            // columns of the neighbouring windows (own column at the block ends)
+  uint32_t xs4;
+  int top;                   // of the block
+};
+__device__ __forceinline__ ResCta& res_cta() { return *reinterpret_cast<ResCta*>(res_smem); }
+template <int NT>
+__device__ __forceinline__ ushort4* res_window() {
+  const ResCta& c = *reinterpret_cast<const ResCta*>(res_smem);
+  return reinterpret_cast<ushort4*>(c.slot + (16 * c.rows8 + 22) * 16 * NT);
+}
+// word `i` of the per-thread words
+template <int NT>
+__device__ __forceinline__ int* res_word(int i) {
+  return reinterpret_cast<int*>(res_smem + kResHead + 4 * NT * i);
+}
+constexpr int kWordPar = 0;   // the largest log2 parity weight; infinite: the block is left to the second pass
+constexpr int kWordExt = 1, kWordMass = 2, kWordSyn = 3;  // largest extrinsic, smallest mass, CRC
+constexpr int kSecondPass = 0x7f800000;
+template <int NT>
+__device__ __forceinline__ char* res_x() {
+  return res_smem + res_x_at(NT);
+}
+template <int NT>
+__device__ __forceinline__ ResWin res_win() {
+  const ResCta& c = res_cta();
+  const ushort4 t = res_window<NT>()[threadIdx.x];
+  ResWin v;
+  v.tid = threadIdx.x;
+  v.k = t.x;
+  v.window = t.y;
+  v.nwin = t.z;
+  v.lane0 = t.w;
+  v.w = v.tid - v.lane0;
+  v.lo = v.w * v.window;
+  v.len = min(v.window, v.k - v.lo);
+  v.guard = c.guard;
+  v.prev = v.w > 0 ? v.tid - 1 : v.tid;
+  v.next = v.w + 1 < v.nwin ? v.tid + 1 : v.tid;
+  v.xs4 = c.xs4;
+  v.top = res_top(__int_as_float(res_word<NT>(kWordPar)[v.lane0]));
+  return v;
+}
+
+__device__ __forceinline__ float lds(const char* x, uint32_t off) {
+  return *reinterpret_cast<const float*>(x + off);
+}
+
+// The scratch slot of the CTA, addressed by 32-bit byte offsets.  Plain loads and stores: what other
+// lanes wrote is read after a barrier, never through the read-only path.
+template <int NT>
+struct Slot {
+  static constexpr uint32_t kPlane = 16u * NT;
+  char* base;
+  uint32_t rows8;
+  __device__ __forceinline__ Slot() : base(res_cta().slot), rows8(res_cta().rows8) {}
+  // byte offset of an 8-step record of the upper / lower SISO, of the checkpoint of such a group, of
+  // the seeds of a SISO written in iterations of a parity, of a SISO's tail
+  static constexpr uint32_t kRecord = 5 * kPlane;
+  __device__ __forceinline__ uint32_t record(bool lower, int g) const {
+    return (lower ? rows8 : 0) * kRecord + g * kRecord;
+  }
+  __device__ __forceinline__ uint32_t ckpt(int g) const { return (10 * rows8 + 2 * g) * kPlane; }
+  // (linear pass) what the last half-iteration read, 8 steps
+  __device__ __forceinline__ uint32_t kept(int g) const { return (12 * rows8 + 2 * g) * kPlane; }
+  __device__ __forceinline__ uint32_t seeds(bool lower, int it) const {
+    return (16 * rows8 + 2 + (lower ? 8 : 0) + (it & 1 ? 4 : 0)) * kPlane;
+  }
+  __device__ __forceinline__ uint32_t tail(bool lower) const {
+    return (16 * rows8 + 18 + (lower ? 2 : 0)) * kPlane;
+  }
+  // planes of a record
+  static constexpr uint32_t kIndex = 2 * kPlane;
+  static constexpr uint32_t kSys = 3 * kPlane;
+  __device__ __forceinline__ float4 ld(uint32_t o) const { return *reinterpret_cast<const float4*>(base + o); }
+  __device__ __forceinline__ uint2 ld2(uint32_t o) const { return *reinterpret_cast<const uint2*>(base + o); }
+  __device__ __forceinline__ void st(uint32_t o, float4 v) const { *reinterpret_cast<float4*>(base + o) = v; }
+  __device__ __forceinline__ void st2(uint32_t o, uint2 v) const { *reinterpret_cast<uint2*>(base + o) = v; }
+  __device__ __forceinline__ void ld8(uint32_t o, float (&v)[8]) const {
+    const float4 x = ld(o), y = ld(o + kPlane);
+    v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
+  }
+  __device__ __forceinline__ void st8(uint32_t o, const float (&v)[8]) const {
+    st(o, make_float4(v[0], v[1], v[2], v[3]));
+    st(o + kPlane, make_float4(v[4], v[5], v[6], v[7]));
+  }
+  // offset of 4 steps' entry within a stream of 2 planes per record
+  static __device__ __forceinline__ uint32_t half(int r) { return (r >> 2 & 1) * kPlane; }
+  // shared-memory offsets of the 4 positions from row r of a column
+  __device__ __forceinline__ uint2 positions(bool lower, int r, int col) const {
+    return ld2(record(lower, r >> 3) + kIndex + 16 * col + ((r & 4) << 1));
+  }
+};
+
+__device__ __forceinline__ void put(float (&b)[8], float4 x, float4 y) {
+  b[0] = x.x; b[1] = x.y; b[2] = x.z; b[3] = x.w; b[4] = y.x; b[5] = y.y; b[6] = y.z; b[7] = y.w;
+}
+
+// The ring: requests go round the stages in order, and so do the reads.
+template <int NT>
+struct Ring {
+  static constexpr uint32_t kStage = 16u * NT * kEntries;
+  uint32_t smem, first, at;  // shared-memory address of res_smem; the thread's entry in stage 0 and in
+                             // the next stage, bytes from there
+  __device__ __forceinline__ Ring() {
+    smem = static_cast<uint32_t>(__cvta_generic_to_shared(res_smem));
+    first = res_ring_at(NT) + 16u * threadIdx.x;
+    at = first;
+  }
+  // requests the parity planes and the positions of the record at `src` into the stage at `to`
+  __device__ __forceinline__ void request(uint32_t to, const char* src, bool any) const {
+    if (any) {
+      to += smem;
+      copy(to, src);
+      copy(to + 16u * NT, src + 16 * NT);
+      copy(to + 32u * NT, src + 32 * NT);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  static __device__ __forceinline__ void copy(uint32_t to, const char* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to), "l"(src) : "memory");
+  }
+  __device__ __forceinline__ void wait() const {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 1) : "memory");
+  }
+  __device__ __forceinline__ float4 ld(int entry) const {
+    return *reinterpret_cast<const float4*>(res_smem + at + 16u * NT * entry);
+  }
+  __device__ __forceinline__ void advance() {
+    at += kStage;
+    if (at == first + kStages * kStage) at = first;
+  }
+  // The inputs of the 8 steps in the next stage: their places in X (w: 8 x uint16 byte offsets), the
+  // LLRs s there, the parities b.
+  __device__ __forceinline__ uint4 read(const char* X, float (&s)[8], float (&b)[8]) const {
+    wait();
+    const float4 q = ld(2);
+    const uint4 w = make_uint4(__float_as_uint(q.x), __float_as_uint(q.y), __float_as_uint(q.z), __float_as_uint(q.w));
+#pragma unroll
+    for (int t = 0; t < 8; ++t) s[t] = lds(X, place(w, t));
+    put(b, ld(0), ld(1));
+    return w;
+  }
+  static __device__ __forceinline__ uint32_t place(const uint4& w, int t) {
+    const uint32_t q = t < 2 ? w.x : t < 4 ? w.y : t < 6 ? w.z : w.w;
+    return t & 1 ? q >> 16 : q & 0xffffu;
+  }
+};
+
+// One SISO half-iteration of one window in the linear domain, first part: everything that reads
+// other windows' positions of X.  Leaves the alpha checkpoints and the next window's alpha seed,
+// and beta at the window's end in `be`.
+template <bool STD, int NT>
+__device__ __forceinline__ void lin_read(const ResWin& v, const Slot<NT>& m, const int it, const bool lower,
+                                         float (&be)[8]) {
+  constexpr uint32_t kPlane = Slot<NT>::kPlane;
+  constexpr uint32_t kRecord = Slot<NT>::kRecord;
+  const char* const X = res_x<NT>();
+  const int tid = v.tid, G = v.guard;
+  const uint32_t seed_in = m.seeds(lower, it), seed_out = m.seeds(lower, it + 1);
+  float al[8];
+  // ---- alpha: warm-up over the last `guard` steps of the previous window, then the window ----
+  {
+    const int gl = v.len >> 3;
+    int j = v.nwin > 1 ? -(G >> 3) : 0;  // 8-step group; negative in the warm-up
+    const int row0 = j < 0 ? v.window - G : 0, col0 = j < 0 ? v.prev : tid;
+    uint32_t ck = m.ckpt(0) + 16u * tid;
+    // i, src: the group that is requested next (the window's own first one follows the warm-up's last)
+    Ring<NT> ring;
+    int i = j;
+    const char* const own = m.base + m.record(lower, 0) + 16u * tid;
+    const char* src = m.base + m.record(lower, row0 >> 3) + 16u * col0;
+    auto request = [&](uint32_t to) {
+      ring.request(to, src, i < gl);
+      src = ++i == 0 ? own : src + kRecord;
+    };
+#pragma unroll
+    for (int st = 0; st < kStages; ++st) request(ring.at + st * Ring<NT>::kStage);
+    if (v.lo - G > 0) {
+      float sd[8];
+      m.ld8(seed_in + 16 * tid, sd);
+      lin_from_log(sd, al, v.top);
+    } else {
+#pragma unroll
+      for (int n = 0; n < 8; ++n) al[n] = n == 0 ? 1.0f : 0.0f;
+    }
+#pragma unroll 1
+    for (; j < gl; ++j) {
+      if (j == 0 && v.w == 0) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) al[k] = k == 0 ? 1.0f : 0.0f;
+      }
+      float s[8], b[8];
+      ring.read(X, s, b);
+      const float r = rescale(al, v.top);
+#pragma unroll
+      for (int n = 0; n < 8; ++n) al[n] *= r;
+      if (j >= 0) {
+        m.st8(ck, al);
+        ck += 2 * kPlane;
+      }
+      request(ring.at);
+      ring.advance();
+#pragma unroll
+      for (int t = 0; t < 8; ++t) alpha_next<STD>(al, weights(s[t], b[t]));
+    }
+  }
+  const int tail_at = v.k - (v.lo + v.len);  // steps of the block behind the window
+  // ---- beta: warm-up over the first `guard` steps of the next window ----
+  float tb[8];
+  m.ld8((tail_at <= G ? m.tail(lower) : seed_in + 2 * kPlane) + 16 * tid, tb);
+  const bool seed_next = v.w + 1 < v.nwin;
+  if (seed_next) {  // the next window's alpha seed: alpha at hi - guard
+    float sd[8];
+    if (G > 0) m.ld8(m.ckpt((v.len - G) >> 3) + 16 * tid, al);
+    log_from_lin(al, sd);
+    m.st8(seed_out + 16 * v.next, sd);
+  }
+  lin_from_log(tb, tb, v.top);
+#pragma unroll
+  for (int n = 0; n < 8; ++n) be[n] = tb[n];
+  if (v.nwin > 1 && G > 0) {
+    Ring<NT> ring;
+    int j = (G >> 3) - 1, i = j;
+    const char* src = m.base + m.record(lower, j) + 16u * v.next;
+    auto request = [&](uint32_t to) {
+      ring.request(to, src, i >= 0);
+      --i;
+      src -= kRecord;
+    };
+#pragma unroll
+    for (int st = 0; st < kStages; ++st) request(ring.at + st * Ring<NT>::kStage);
+#pragma unroll 1
+    for (; j >= 0; --j) {
+      if (8 * (j + 1) == tail_at) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) be[k] = tb[k];
+      }
+      float s[8], b[8];
+      ring.read(X, s, b);
+      request(ring.at);
+      ring.advance();
+      const float r = rescale(be, v.top);
+#pragma unroll
+      for (int t = 7; t >= 0; --t) beta_next<STD>(be, weights(s[t], b[t]), t == 7 ? r : 1.0f);
+    }
+    if (tail_at == 0) {
+#pragma unroll
+      for (int n = 0; n < 8; ++n) be[n] = tb[n];
+    }
+  }
+}
+
+// Second part, 8 steps at a time, last to first: alpha recomputed from its checkpoint, beta and the
+// extrinsic; the previous window's beta seed is beta at lo + guard.  Replaces the LLRs of the
+// window's own positions in X by the other SISO's input Ls + extrinsic, or (post) by the posterior;
+// with keep_ext the extrinsics stay in the checkpoint planes too, with keep what was read (should a
+// check fail).  Returns the largest |x|
+// and the smallest mass of all paths (0: an overflow or a NaN).
+template <bool STD, int NT>
+__device__ __forceinline__ float2 lin_write(const ResWin& v, const Slot<NT>& m, const int it, const bool lower,
+                                          float (&be)[8], const float scale, const bool post,
+                                          const bool keep_ext, const bool keep) {
+  constexpr uint32_t kPlane = Slot<NT>::kPlane;
+  constexpr uint32_t kRecord = Slot<NT>::kRecord;
+  char* const X = res_x<NT>();
+  const int tid = v.tid, G = v.guard;
+  const uint32_t seed_out = m.seeds(lower, it + 1) + 2 * kPlane + 16 * v.prev;
+  float xmax = 0.0f, smax = 0.0f, mass = 3.0e38f;  // checks
+  const bool rec = v.w > 0 && G <= v.len;
+  Ring<NT> ring;
+  int j = (v.len >> 3) - 1, i = j;
+  const char* src = m.base + m.record(lower, j) + 16u * tid;
+  const char* ls = src + Slot<NT>::kSys;
+  char* ck = m.base + m.ckpt(j) + 16u * tid;
+  const uint32_t kept = m.kept(0) - m.ckpt(0);
+  auto request = [&](uint32_t to) {
+    ring.request(to, src, i >= 0);
+    --i;
+    src -= kRecord;
+  };
+#pragma unroll
+  for (int st = 0; st < kStages; ++st) request(ring.at + st * Ring<NT>::kStage);
+  auto ld = [](const char* p) { return *reinterpret_cast<const float4*>(p); };
+  float4 ca = ld(ck), cb = ld(ck + kPlane), la = ld(ls), lb = ld(ls + kPlane);
+  if (rec && v.len == G) {
+    float sd[8];
+    log_from_lin(be, sd);
+    m.st8(seed_out, sd);
+  }
+#pragma unroll 1
+  for (; j >= 0; --j) {
+    float s[8], b[8], a[8], base[8];
+    const uint4 places = ring.read(X, s, b);
+    put(a, ca, cb);
+    put(base, la, lb);
+    if (post) {
+#pragma unroll
+      for (int t = 0; t < 8; ++t) base[t] = s[t];
+    }
+    request(ring.at);
+    ring.advance();
+    char* const here = ck;
+    if (keep) {
+      *reinterpret_cast<float4*>(here + kept) = make_float4(s[0], s[1], s[2], s[3]);
+      *reinterpret_cast<float4*>(here + kept + kPlane) = make_float4(s[4], s[5], s[6], s[7]);
+    }
+    if (j > 0) {
+      ck -= 2 * kPlane;
+      ls -= kRecord;
+      ca = ld(ck);
+      cb = ld(ck + kPlane);
+      la = ld(ls);
+      lb = ld(ls + kPlane);
+    }
+    Weights wt[8];
+#pragma unroll
+    for (int t = 0; t < 8; ++t) wt[t] = weights(s[t], b[t]);
+    const float rb = rescale(be, v.top);
+    // A[t]: alpha_{t+1} without its input weight (reference code) or alpha_t (TS 36.212)
+    float A[8][8];
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+      if constexpr (STD) {
+#pragma unroll
+        for (int n = 0; n < 8; ++n) A[t][n] = a[n];
+        if (t < 7) alpha_next<STD>(a, wt[t]);
+      } else {
+        alpha_lin(a, wt[t].b, A[t]);
+        if (t < 7) input_scale(A[t], wt[t].a1, wt[t].a0, a);
+      }
+    }
+    float e[8], xl = 0.0f;
+#pragma unroll
+    for (int t = 7; t >= 0; --t) {
+      float s1, s0;
+      if constexpr (STD) {
+        // sums over the branches of each input and parity
+        float z[2][2] = {{0.0f, 0.0f}, {0.0f, 0.0f}};
+#pragma unroll
+        for (int n = 0; n < 8; ++n) {
+          const int p0 = 2 * (n & 3);
+          float& x0 = z[pred_input<true>(n, 0)][pred_parity(n, 0)];
+          x0 = fmaf(A[t][p0], be[n], x0);
+          float& x1 = z[pred_input<true>(n, 1)][pred_parity(n, 1)];
+          x1 = fmaf(A[t][p0 + 1], be[n], x1);
+        }
+        s1 = fmaf(wt[t].b, z[1][1], z[1][0]);
+        s0 = fmaf(wt[t].b, z[0][1], z[0][0]);
+      } else {
+        // states entered with input 1: {1, 2, 4, 7}; with input 0: {0, 3, 5, 6}
+        s1 = A[t][1] * be[1];
+        s0 = A[t][0] * be[0];
+        s1 = fmaf(A[t][2], be[2], s1);
+        s0 = fmaf(A[t][3], be[3], s0);
+        s1 = fmaf(A[t][4], be[4], s1);
+        s0 = fmaf(A[t][5], be[5], s0);
+        s1 = fmaf(A[t][7], be[7], s1);
+        s0 = fmaf(A[t][6], be[6], s0);
+      }
+      const float x = log_ratio(s1, s0);
+      if (t & 1) xl = x;
+      else xmax = max3(xmax, fabsf(x), fabsf(xl));
+      smax = max3_nan(smax, s1, s0);
+      if (t == 0) mass = min_nan(mass, fmaf(wt[t].a1, s1, wt[t].a0 * s0));
+      e[t] = scale * x;
+      *reinterpret_cast<float*>(X + Ring<NT>::place(places, t)) = base[t] + e[t];
+      if (keep_ext && (t & 3) == 0)
+        *reinterpret_cast<float4*>(here + (t >> 2) * kPlane) = make_float4(e[t], e[t + 1], e[t + 2], e[t + 3]);
+      beta_next<STD>(be, wt[t], t == 7 ? rb : 1.0f);
+    }
+    // input weights flushed to 0: |s| > 126, less the log of b, which is up to 108 - 2 top
+    const float smag = max3(max3(fabsf(s[0]), fabsf(s[1]), fabsf(s[2])), max3(fabsf(s[3]), fabsf(s[4]), fabsf(s[5])),
+                            fmaxf(fabsf(s[6]), fabsf(s[7])));
+    if (!(smag <= 2.0f * v.top)) {
+#pragma unroll
+      for (int t = 0; t < 8; ++t)
+        if (fminf(wt[t].a1, wt[t].a0) == 0.0f)
+          mass = min_nan(mass, ex2((s[t] < 0.0f ? -e[t] : e[t]) / scale + static_cast<float>(v.top) + (126.0f - kKept - kLost)));
+    }
+    if (rec && 8 * j == G) {
+      float sd[8];
+      log_from_lin(be, sd);
+      m.st8(seed_out, sd);
+    }
+  }
+  return make_float2(xmax, smax < 0x1p126f && mass > 0.0f ? mass : 0.0f);
+}
+
+// A half-iteration of the CTA's blocks in the linear domain; `run`: this thread's window takes part.
+// Returns the bits by which its block passed the checks (negative: it did not).
+template <bool STD, int NT>
+__device__ __noinline__ float lin_half(const bool run, const int half, const float scale, const bool post,
+                                       const bool keep_ext, const bool keep) {
+  const ResWin v = res_win<NT>();
+  const Slot<NT> m;
+  const bool lower = half & 1;
+  float be[8];
+  if (run) lin_read<STD, NT>(v, m, half >> 1, lower, be);
+  __syncthreads();  // every window has read X (and left its seeds and checkpoints)
+  float2 c = make_float2(0.0f, 0.0f);
+  if (run) c = lin_write<STD, NT>(v, m, half >> 1, lower, be, scale, post, keep_ext, keep);
+  __syncthreads();
+  res_word<NT>(kWordExt)[threadIdx.x] = 0;
+  res_word<NT>(kWordMass)[threadIdx.x] = 0x7f000000;
+  __syncthreads();
+  if (run) {
+    atomicMax(res_word<NT>(kWordExt) + v.lane0, __float_as_int(c.x));
+    atomicMin(res_word<NT>(kWordMass) + v.lane0, __float_as_int(c.y));
+  }
+  __syncthreads();
+  return lg2(__int_as_float(res_word<NT>(kWordMass)[v.lane0])) - __int_as_float(res_word<NT>(kWordExt)[v.lane0]) -
+         (static_cast<float>(v.top) - kLost);
+}
+
+// The extrinsics in the checkpoint planes into X: added to Ls (the other SISO's input), or (post)
+// to what stands there (the posterior).
+template <int NT>
+__device__ __noinline__ void put_extrinsics(const bool lower, const bool post) {
+  const ResWin v = res_win<NT>();
+  const Slot<NT> m;
+  char* const X = res_x<NT>();
+  // 32 steps at a time, all loads before any use (rows behind the window repeat its last ones)
+  constexpr int kPart = 4;
+#pragma unroll 1
+  for (int r0 = 0; r0 < v.len; r0 += 8 * kPart) {
+    float e[kPart][8], l[kPart][8];
+    uint4 q[kPart];
+#pragma unroll
+    for (int i = 0; i < kPart; ++i) {
+      const int g = min(r0 + 8 * i, v.len - 8) >> 3;
+      m.ld8(m.ckpt(g) + 16 * v.tid, e[i]);
+      m.ld8(m.record(lower, g) + m.kSys + 16 * v.tid, l[i]);
+      q[i] = *reinterpret_cast<const uint4*>(m.base + m.record(lower, g) + m.kIndex + 16 * v.tid);
+    }
+#pragma unroll
+    for (int i = 0; i < kPart; ++i) {
+      if (r0 + 8 * i >= v.len) break;
+#pragma unroll
+      for (int t = 0; t < 8; ++t) {
+        float* d = reinterpret_cast<float*>(X + Ring<NT>::place(q[i], t));
+        *d = (post ? *d : l[i][t]) + e[i][t];
+      }
+    }
+  }
+}
+
+// Taped forward pass: what a half-iteration of this thread's window reads, log2(e) (Ls + La) in the
+// SISO's order and the seeds.
+template <int NT>
+__device__ __noinline__ void res_tape(const Tape& t, const int cb, const int half, const float unit) {
+  const ResWin v = res_win<NT>();
+  const Slot<NT> m;
+  const bool lower = half & 1;
+  const char* const X = res_x<NT>();
+  const DevCb& d = t.cbs[cb];
+  float* o = t.s + half * t.stride + d.work + v.lo;
+#pragma unroll 2
+  for (int r = 0; r < v.len; r += 8, o += 8) {
+    const uint4 q = *reinterpret_cast<const uint4*>(m.base + m.record(lower, r >> 3) + m.kIndex + 16 * v.tid);
+    float s[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) s[k] = unit * lds(X, Ring<NT>::place(q, k));
+    *reinterpret_cast<float4*>(o) = make_float4(s[0], s[1], s[2], s[3]);
+    *reinterpret_cast<float4*>(o + 4) = make_float4(s[4], s[5], s[6], s[7]);
+  }
+  float4* const sd = reinterpret_cast<float4*>(t.seeds + half * t.slab + 16 * static_cast<int64_t>(d.win0 + v.w));
+#pragma unroll
+  for (int k = 0; k < 4; ++k) sd[k] = m.ld(m.seeds(lower, half >> 1) + k * m.kPlane + 16 * v.tid);
+}
+
+// X of this thread's window as the half-iteration that failed had it, in natural units.
+template <int NT>
+__device__ __noinline__ void res_restore(const bool lower) {
+  const ResWin v = res_win<NT>();
+  const Slot<NT> m;
+  char* const X = res_x<NT>();
+#pragma unroll 2
+  for (int g = 0; g < v.len >> 3; ++g) {
+    float s[8];
+    m.ld8(m.kept(g) + 16 * v.tid, s);
+    const uint4 q = *reinterpret_cast<const uint4*>(m.base + m.record(lower, g) + m.kIndex + 16 * v.tid);
+#pragma unroll
+    for (int t = 0; t < 8; ++t) *reinterpret_cast<float*>(X + Ring<NT>::place(q, t)) = kLn2 * s[t];
+  }
+}
+
+// A warp's windows by block: calls f(lane of the block's first window in this warp, steps) for each
+// block (its windows in a warp are consecutive lanes, their steps consecutive in every stream).
+template <class F>
+__device__ __forceinline__ void res_for_blocks(const ResWin& v, F f) {
+  const int lane = threadIdx.x & 31;
+  unsigned first = __ballot_sync(0xffffffffu, v.len > 0 && (v.w == 0 || lane == 0));
+  while (first) {
+    const int l = __ffs(first) - 1;
+    first &= first - 1;
+    // up to the block's end, or to the end of the warp's last lane
+    const int k = __shfl_sync(0xffffffffu, v.k, l), lo = __shfl_sync(0xffffffffu, v.lo, l);
+    f(l, min(k - lo, (32 - l) * __shfl_sync(0xffffffffu, v.window, l)), __shfl_sync(0xffffffffu, v.window, l));
+  }
+}
+
+// Copies the windows' rows (entries of SIZE bytes; `src`: this lane's window) to stage + thread *
+// pitch, each warp its own with consecutive 16-byte pieces per lane, and waits for them.
+template <int SIZE>
+__device__ __forceinline__ void res_stage_rows(const ResWin& v, const void* src, char* stage, int pitch) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t to = static_cast<uint32_t>(__cvta_generic_to_shared(stage)) + (threadIdx.x & ~31) * pitch;
+  constexpr int kPiece = 16 / SIZE;
+  res_for_blocks(v, [&](int l, int steps, int window) {
+    const char* p = reinterpret_cast<const char*>(
+        __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(src), l));
+    const uint32_t inv = 0xffffffffu / static_cast<uint32_t>(window) + 1u;
+#pragma unroll 4
+    for (int q = kPiece * lane; q < steps; q += kPiece * 32) {
+      const int w = __umulhi(q, inv);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + (l + w) * pitch + (q - w * window) * SIZE),
+                   "l"(p + q * SIZE)
+                   : "memory");
+    }
+  });
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncwarp();
+}
+
+// The inputs of a task, in base-2 units with parity weights for the linear pass: the streams' planes, X = the systematic LLRs (the first input of
+// the upper SISO), the interleaved positions, the tail betas, seeds zero.
+// Each warp stages its windows' rows through shared memory (where X and the ring will be; a row
+// pitch of an odd number of 16-byte words keeps both sides free of bank conflicts).
+template <bool STD, int NT>
+__device__ __noinline__ void res_inputs(const ResCb* cb, const float* llr, const uint16_t* perm,
+                                        const bool linear) {
+  const Slot<NT> m;
+  const float unit = linear ? kLog2e : 1.0f;
+  const int tid = threadIdx.x;
+  const bool mine = cb != nullptr;
+  const ResWin v = res_win<NT>();
+  char* const X = res_x<NT>();
+  char* const stage = res_smem + res_ring_at(NT);
+  const int W = res_cta().max_window;
+  const float* const d0 = mine ? llr + cb->llr : nullptr;
+  __syncthreads();
+  {  // positions: rows of uint16
+    const int pitch = 2 * W + 16;
+    // a row starts at any multiple of 8 entries: 16-byte aligned
+    res_stage_rows<2>(v, mine ? perm + cb->tab + v.lo : nullptr, stage, pitch);
+    if (mine) {
+      const uint32_t inv = 0xffffffffu / static_cast<uint32_t>(v.window) + 1u;
+      const char* row = stage + tid * pitch;
+#pragma unroll 2
+      for (int r = 0; r < v.window; r += 8) {
+        uint32_t o[8];
+        if (r < v.len) {
+          const uint4 q = *reinterpret_cast<const uint4*>(row + 2 * r);
+          const uint32_t n[8] = {q.x & 0xffffu, q.x >> 16, q.y & 0xffffu, q.y >> 16,
+                                 q.z & 0xffffu, q.z >> 16, q.w & 0xffffu, q.w >> 16};
+#pragma unroll
+          for (int t = 0; t < 8; ++t) {
+            const uint32_t w = __umulhi(n[t], inv);
+            o[t] = (n[t] - w * v.window) * v.xs4 + 4u * (v.lane0 + w);
+          }
+        } else {  // behind the block's last step: any place
+#pragma unroll
+          for (int t = 0; t < 8; ++t) o[t] = 4u * tid;
+        }
+        *reinterpret_cast<uint4*>(m.base + m.record(true, r >> 3) + m.kIndex + 16u * tid) =
+            make_uint4(o[0] | o[1] << 16, o[2] | o[3] << 16, o[4] | o[5] << 16, o[6] | o[7] << 16);
+        const uint32_t own = r * v.xs4 + 4u * tid, two = own | own << 16, step = v.xs4 | v.xs4 << 16;
+        *reinterpret_cast<uint4*>(m.base + m.record(false, r >> 3) + m.kIndex + 16u * tid) =
+            make_uint4(two + (v.xs4 << 16), two + 2 * step + (v.xs4 << 16), two + 4 * step + (v.xs4 << 16),
+                       two + 6 * step + (v.xs4 << 16));
+      }
+    }
+    __syncwarp();
+  }
+  const int pitch = 4 * W + 16;
+#pragma unroll 1
+  for (int st = 0; st < 3; ++st) {  // parity 1, parity 2, systematic
+    const int which = st == 2 ? 0 : st + 1;
+    if (NT > 32) __syncthreads();  // (pitches differ: a row may lie in another warp's part)
+    res_stage_rows<4>(v, mine ? d0 + which * (v.k + 4) + v.lo : nullptr, stage, pitch);
+    if (mine) {
+      const char* row = stage + tid * pitch;
+      float most = 0.0f;
+      const bool exp_now = linear && which != 0;
+#pragma unroll 4
+      for (int r = 0; r < v.window; r += 4) {
+        float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (r < v.len) x = *reinterpret_cast<const float4*>(row + 4 * r);
+        most = fmaxf(max3(most, x.x, x.y), fmaxf(x.z, x.w));
+        x = make_float4(unit * x.x, unit * x.y, unit * x.z, unit * x.w);
+        if (exp_now) x = make_float4(ex2(x.x), ex2(x.y), ex2(x.z), ex2(x.w));
+        m.st(m.record(which == 2, r >> 3) + (which == 0 ? m.kSys : 0) + m.half(r) + 16u * tid, x);
+      }
+      if (which != 0) atomicMax(res_word<NT>(kWordPar) + v.lane0, __float_as_int(unit * most));
+    }
+    __syncwarp();
+  }
+  __syncthreads();
+  if (mine) {
+    // 32 steps at a time, all loads before any store
+#pragma unroll 1
+    for (int r0 = 0; r0 < v.len; r0 += 32) {
+      float4 x[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int r = min(r0 + 4 * i, v.len - 4);
+        x[i] = m.ld(m.record(false, r >> 3) + m.kSys + m.half(r) + 16 * tid);
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if (r0 + 4 * i >= v.len) break;
+        char* d = X + (r0 + 4 * i) * v.xs4 + 4 * tid;
+        *reinterpret_cast<float*>(d) = x[i].x;
+        *reinterpret_cast<float*>(d + v.xs4) = x[i].y;
+        *reinterpret_cast<float*>(d + 2 * v.xs4) = x[i].z;
+        *reinterpret_cast<float*>(d + 3 * v.xs4) = x[i].w;
+      }
+    }
+  }
+  __syncthreads();
+  if (!mine) return;
+#pragma unroll 1
+  for (int r0 = 0; r0 < v.window; r0 += 32) {
+    uint4 q[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      q[i] = *reinterpret_cast<const uint4*>(
+          m.base + m.record(true, min(r0 + 8 * i, v.window - 8) >> 3) + m.kIndex + 16u * tid);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (r0 + 8 * i >= v.window) break;
+      const uint32_t at = m.record(true, (r0 >> 3) + i) + m.kSys + 16u * tid;
+      m.st(at, make_float4(lds(X, q[i].x & 0xffffu), lds(X, q[i].x >> 16), lds(X, q[i].y & 0xffffu),
+                           lds(X, q[i].y >> 16)));
+      m.st(at + m.kPlane, make_float4(lds(X, q[i].z & 0xffffu), lds(X, q[i].z >> 16),
+                                      lds(X, q[i].w & 0xffffu), lds(X, q[i].w >> 16)));
+    }
+  }
+  const uint32_t sd = m.seeds(false, 0) + 16u * tid;
+#pragma unroll 1
+  for (int i = 0; linear && i < 16; ++i) m.st(sd + i * m.kPlane, make_float4(0.0f, 0.0f, 0.0f, 0.0f));
+  if (v.k - (v.lo + v.len) <= v.guard) {
+#pragma unroll
+    for (int lower = 0; lower < 2; ++lower) {
+      float ts[3], tp[3], tb[8];
+      tail_llrs<STD>(lower, d0, v.k, ts, tp);
+      tail_beta<STD>(tb, ts, tp);
+      m.st8(m.tail(lower) + 16u * tid, tb);
+    }
+  }
+}
+
+// This window's part of its block's CRC24B syndrome of the hard decisions [filler, K)
+// (lte_turbo.cpp:792-804): the window's bits modulo g 4 at a time, times x^(steps behind it).
+template <int NT>
+__device__ __noinline__ void res_crc(const uint32_t* xpow, const int filler) {
+  const ResWin v = res_win<NT>();
+  const char* const X = res_x<NT>();
+  const uint32_t* const tab = res_cta().crc_tab;
+  uint32_t c = 0, off = 4u * v.tid;
+#pragma unroll 4
+  for (int r = 0; r < v.len; r += 8) {
+    uint32_t byte = 0;
+#pragma unroll
+    for (int t = 0; t < 8; ++t, off += v.xs4) {
+      const bool bit = lds(X, off) >= 0.0f && v.lo + r + t >= filler;
+      byte = 2 * byte + (bit ? 1u : 0u);
+    }
+    c = ((c << 4) & 0xffffffu) ^ tab[c >> 20] ^ (byte >> 4);
+    c = ((c << 4) & 0xffffffu) ^ tab[c >> 20] ^ (byte & 15u);
+  }
+  uint32_t z = 0;
+  const uint32_t* xp = xpow + (v.k - (v.lo + v.len));
+#pragma unroll
+  for (int b = 0; b < 24; ++b) z ^= (c >> b) & 1u ? __ldg(xp + b) : 0u;
+  atomicXor(reinterpret_cast<uint32_t*>(res_word<NT>(kWordSyn)) + v.lane0, z);
+}
+
+// The posteriors in X, times `unit`, of the windows whose lane has a `dst` to there, each warp its own
+// windows.
+template <int NT>
+__device__ __noinline__ void res_outputs(float* dst, const float unit) {
+  const ResWin v = res_win<NT>();
+  const int lane = threadIdx.x & 31;
+  const char* const X = res_x<NT>() + 4 * (v.tid - lane);
+  res_for_blocks(v, [&](int l, int steps, int window) {
+    float* const p = reinterpret_cast<float*>(
+        __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(dst), l));
+    if (p == nullptr) return;
+    const uint32_t inv = 0xffffffffu / static_cast<uint32_t>(window) + 1u;
+#pragma unroll 8
+    for (int q = lane; q < steps; q += 32) {
+      const int w = __umulhi(q, inv);
+      p[q] = unit * lds(X, (q - w * window) * v.xs4 + 4u * (l + w));
+    }
+  });
+}
+
+// ---- second pass: blocks whose metrics left float's range, in the (m, s) form of siso.cuh, with
+// X and the planes in natural units ----
+template <bool LOWER, int NT>
+struct SlotAccess {
+  ResWin v;
+  Slot<NT> m;
+  uint32_t seed_in, seed_out;
+  float factor;
+  const float* d0;
+  __device__ __forceinline__ int guard() const { return v.guard; }
+  __device__ __forceinline__ float scale() const { return factor; }
+  // 4 steps from q (of the block), which may lie in a neighbouring window
+  __device__ __forceinline__ Raw4 raw4(int q) const {
+    int row = q - v.lo, col = v.tid;
+    if (row < 0) {
+      row += v.window;
+      --col;
+    } else if (row >= v.window) {
+      row -= v.window;
+      ++col;
+    }
+    const char* const X = res_x<NT>();
+    const uint2 w = m.positions(LOWER, row, col);
+    return Raw4{make_float4(lds(X, w.x & 0xffffu), lds(X, w.x >> 16), lds(X, w.y & 0xffffu), lds(X, w.y >> 16)),
+                make_float4(0.0f, 0.0f, 0.0f, 0.0f),
+                m.ld(m.record(LOWER, row >> 3) + m.half(row) + 16 * col)};
+  }
+  __device__ __forceinline__ Raw8 raw8(int q) const { return Raw8{raw4(q), raw4(q + 4)}; }
+  __device__ __forceinline__ void load_seed(bool beta, float (&x)[8]) const {
+    m.ld8(seed_in + (beta ? 2 * m.kPlane : 0) + 16 * v.tid, x);
+  }
+  __device__ __forceinline__ void store_seed(bool beta, const float (&x)[8]) const {
+    m.st8(seed_out + (beta ? 2 * m.kPlane + 16 * v.prev : 16 * v.next), x);
+  }
+  __device__ __forceinline__ uint2 targets(int) const { return make_uint2(0, 0); }
+  __device__ __forceinline__ void put(int q, int, float e, float) const {
+    const int row = q - v.lo;
+    *reinterpret_cast<float*>(m.base + m.ckpt(row >> 3) + m.half(row) + 16 * v.tid + 4 * (row & 3)) = e;
+  }
+};
+
+// A half-iteration of this thread's window: reads X, leaves the extrinsics in the checkpoint planes.
+template <bool LOWER, bool STD, int NT>
+__device__ __noinline__ void log_half(const float* d0, const int it, const float scale) {
+  SlotAccess<LOWER, NT> io;
+  io.v = res_win<NT>();
+  io.seed_in = io.m.seeds(LOWER, it);
+  io.seed_out = io.m.seeds(LOWER, it + 1);
+  io.factor = scale;
+  io.d0 = d0;
+  DevCb cb{};
+  cb.k = io.v.k;
+  cb.nwin = io.v.nwin;
+  cb.window = io.v.window;
+  const CkptStrided ck{reinterpret_cast<float4*>(io.m.base) + 12 * io.m.rows8 * NT, NT, io.v.tid};
+  siso_window<kSub, LOWER, STD>(cb, io.v.w, io, ck);
+}
+
+template <bool STD, int NT>
+__global__ void __launch_bounds__(NT, 256 / NT) resident_kernel(const __grid_constant__ ResArgs p) {
+  const int tid = threadIdx.x;
+  ResCta& cta = res_cta();
+  int* const left = res_word<NT>(kWordPar);  // kSecondPass: the block (at its first lane) left the linear domain
+  for (int task = blockIdx.x; task < p.n_tasks;) {
+    if (task == p.stall_task && tid == 0) {  // testing hook: a wait that runs out
+      const uint64_t t0 = global_ns();
+      while (load_acquire(p.never) == 0) {
+        if (global_ns() - t0 > kWaitLimitNs) {
+          atomicExch(p.error, 1);
+          break;
+        }
+        __nanosleep(256);
+      }
+    }
+    const int first = p.task_first[task], last = p.task_first[task + 1];
+    const ResCb* cb = nullptr;  // this thread's block
+    int lane0 = 0, lanes = 0, max_window = 0;
+    ushort4 win = make_ushort4(0, 0, 0, 0);
+    for (int c = first; c < last; ++c) {
+      const ResCb& o = p.cbs[c];
+      const int l0 = o.lane0, n = o.nwin;
+      if (tid >= l0 && tid < l0 + n) {
+        cb = &o;
+        lane0 = l0;
+        win = make_ushort4(o.k, o.window, n, l0);
+      }
+      lanes = l0 + n;
+      max_window = max(max_window, o.window);
+    }
+    const bool mine = cb != nullptr;
+    left[tid] = 0;
+    if (tid == 0) {
+      cta.slot = reinterpret_cast<char*>(p.scratch + p.slot * blockIdx.x);
+      cta.guard = p.guard;
+      cta.rows8 = p.rows8;
+      cta.xs4 = 4u * res_pitch(lanes);
+      cta.max_window = max_window;
+    }
+    if (tid < 16) cta.crc_tab[tid] = __ldg(p.xpow + kXpowSize + tid);
+    __syncthreads();
+    res_window<NT>()[tid] = win;  // read by this thread alone
+    bool passed = false;
+    int used = p.max_iterations;
+
+    // Two passes: all blocks in the linear domain, then the ones that left float's range there, in the
+    // (m, s) form from half-iteration `from`.
+    int from = 0;
+    float margin = 1000.0f;  // of the block's checks in the last half-iteration
+#pragma unroll 1
+    for (int pass = 0; pass < 2 && p.max_iterations > 0; ++pass) {
+      bool run = mine && (pass == 0 || left[lane0] == kSecondPass);
+      if (pass == 1 && !__syncthreads_or(run)) break;
+      const bool taken = run;
+      res_inputs<STD, NT>(cb, p.llr, p.perm, pass == 0);
+      __syncthreads();
+      if (pass == 1) {
+        if (run && from > 0) res_restore<NT>(from & 1);
+        __syncthreads();
+      }
+      if (pass == 0) {
+        const bool wide = run && __int_as_float(left[lane0]) > kMaxParity;
+        __syncthreads();
+        if (wide) {
+          left[lane0] = kSecondPass;
+          run = false;
+        }
+      }
+#pragma unroll 1
+      for (int half = 0; half < 2 * p.max_iterations; ++half) {
+        const int it = half >> 1;
+        const bool lower = half & 1, last_half = half + 1 == 2 * p.max_iterations;
+        const bool post_now = lower && (p.early_stop || last_half);
+        const float scale = __ldg(p.scale + half);
+        if (p.tape.s != nullptr && run && half >= (pass == 0 ? 0 : from)) res_tape<NT>(p.tape, cb->idx, half, pass == 0 ? 1.0f : kLog2e);
+        if (pass == 0) {
+          // (a block that fails is left to the second pass)
+          const bool keep = margin < kNear;
+          margin = lin_half<STD, NT>(run, half, scale, post_now, lower && p.early_stop, keep);
+          if (!(margin >= 0.0f) && run) {
+            left[lane0] = kSecondPass;
+            run = false;
+            from = keep ? half : 0;
+          }
+        } else {
+          if (run && half >= from) {
+            const float* d0 = p.llr + cb->llr;
+            if (lower) log_half<true, STD, NT>(d0, it, scale);
+            else log_half<false, STD, NT>(d0, it, scale);
+          }
+          __syncthreads();
+          if (run && half >= from) put_extrinsics<NT>(lower, post_now);
+        }
+        __syncthreads();
+        if (post_now && p.early_stop) {
+          res_word<NT>(kWordSyn)[tid] = 0;
+          __syncthreads();
+          if (run && half >= from) res_crc<NT>(p.xpow, cb->filler);
+          __syncthreads();
+          if (run && half >= from) {
+            used = it + 1;
+            passed = res_word<NT>(kWordSyn)[lane0] == 0;
+            // X goes from the posterior to the next iteration's input
+            if (!passed && !last_half) put_extrinsics<NT>(true, false);
+            run = !passed;
+          }
+          if (!__syncthreads_or(run)) break;
+        }
+      }
+      const bool write = taken && (pass == 1 || left[lane0] != kSecondPass);
+      res_outputs<NT>(write ? p.post + cb->out + (tid - lane0) * cb->window : nullptr,
+                      pass == 0 ? kLn2 : 1.0f);
+      __syncthreads();
+    }
+    if (mine && tid == lane0) {
+      p.crc_ok[cb->idx] = passed ? 1 : 0;
+      p.iters[cb->idx] = static_cast<uint32_t>(used);
+    }
+    if (p.n_tasks <= static_cast<int>(gridDim.x)) return;
+    __syncthreads();
+    if (tid == 0) cta.next_task = static_cast<int>(gridDim.x) + atomicAdd(p.queue, 1);
+    __syncthreads();
+    task = cta.next_task;
+    __syncthreads();
+  }
+}
+
+}  // namespace
+}  // namespace tcb

@@ -1,5 +1,5 @@
-// siso.cuh -- one window of one SISO half-iteration, shared by the plain (one launch per
-// half-iteration) and the persistent (all iterations in one launch) decoders.
+// siso.cuh -- one window of one SISO half-iteration of the launch-per-half-iteration decoder
+// (windows too long for the block-resident one, the allocation-free entry point).
 //
 // A window [lo, hi) of a code block is owned by one thread, which keeps the 8 state metrics
 // in registers.  Its forward recursion starts `guard` steps before the window and its backward
@@ -10,7 +10,7 @@
 // (decode_siso_log_map, lte_turbo.cpp:410-486).
 //
 // Memory use per thread: the forward pass stores alpha only every S steps (checkpoints, 32 B
-// each, in shared memory or global scratch with the windows of a launch interleaved); the
+// each, in global scratch with the windows of a launch interleaved); the
 // backward pass recomputes the S alphas of one sub-window into registers from its checkpoint
 // and then runs beta + extrinsic over it.  The metrics are in the deferred-log (m, s) form of
 // trellis.cuh.
@@ -19,10 +19,6 @@
 #include <type_traits>
 
 #include "trellis.cuh"
-
-#ifndef TCB_LDCG
-#define TCB_LDCG 0
-#endif
 
 namespace tcb {
 
@@ -51,41 +47,19 @@ struct SisoIo {
   float* seed_out;
   float scale;            // extrinsic scale of this half-iteration (1.0 for the plain decoder)
   int guard;
+  float* tape = nullptr;  // taped forward pass: log2(e) (Ls + La) in this SISO's order (work layout)
 };
 
 __device__ __forceinline__ float4 ld4(const float* p) {
   return __ldg(reinterpret_cast<const float4*>(p));
 }
-// Loads of data written earlier in the same kernel (persistent schedule): an ordinary
-// (coherent, L1-cacheable) global load, never the read-only non-coherent path.  The writer
-// releases and the reader acquires at GPU scope before these loads, which makes them see the
-// writes even when the writer ran on another SM.
-__device__ __forceinline__ float4 ld4_coherent(const float* p) {
-#if TCB_LDCG
-  return __ldcg(reinterpret_cast<const float4*>(p));
-#else
-  float4 v;
-  asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
-               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-               : "l"(p)
-               : "memory");
-  return v;
-#endif
-}
-template <bool COHERENT>
-__device__ __forceinline__ float4 ld4_io(const float* p) {
-  return COHERENT ? ld4_coherent(p) : ld4(p);
-}
-
-// Raw inputs of 4 consecutive steps (one float4 per stream).  The a-priori stream is written
-// by the other SISO; COHERENT reads it through L2 (needed when both run in one kernel).
+// Raw inputs of 4 consecutive steps (one float4 per stream).
 struct Raw4 {
   float4 s, e, p;  // systematic, a-priori, parity
 };
-template <bool COHERENT = false>
 __device__ __forceinline__ Raw4 load_raw4(const float* sys, const float* apr, const float* par,
                                           int q) {
-  return Raw4{ld4(sys + q), ld4_io<COHERENT>(apr + q), ld4(par + q)};
+  return Raw4{ld4(sys + q), ld4(apr + q), ld4(par + q)};
 }
 // raw -> sys+apr (sa), a = c (sys+apr), b = c par with c = log2(e)/2
 __device__ __forceinline__ void scale4(const Raw4& r, float* sa, float* a, float* b) {
@@ -101,40 +75,13 @@ __device__ __forceinline__ void scale4(const Raw4& r, float* sa, float* a, float
 struct Raw8 {
   Raw4 lo, hi;
 };
-template <bool COHERENT = false>
 __device__ __forceinline__ Raw8 load_raw8(const float* sys, const float* apr, const float* par,
                                           int q) {
-  return Raw8{load_raw4<COHERENT>(sys, apr, par, q), load_raw4<COHERENT>(sys, apr, par, q + 4)};
+  return Raw8{load_raw4(sys, apr, par, q), load_raw4(sys, apr, par, q + 4)};
 }
 
-// Checkpoint storage, 8 floats per checkpoint as two float4.  Shared memory: thread-minor
-// float4 planes (conflict-free); global scratch: a per-thread slot.
-struct CkptSmem {
-  float4* base;  // dynamic shared memory
-  int stride;    // threads per block
-  int tid;
-  __device__ __forceinline__ void store(int j, const float (&m)[8]) const {
-    base[(2 * j) * stride + tid] = make_float4(m[0], m[1], m[2], m[3]);
-    base[(2 * j + 1) * stride + tid] = make_float4(m[4], m[5], m[6], m[7]);
-  }
-  __device__ __forceinline__ void load(int j, float (&m)[8]) const {
-    const float4 x = base[(2 * j) * stride + tid], y = base[(2 * j + 1) * stride + tid];
-    m[0] = x.x; m[1] = x.y; m[2] = x.z; m[3] = x.w; m[4] = y.x; m[5] = y.y; m[6] = y.z; m[7] = y.w;
-  }
-};
-struct CkptGlobal {
-  float4* base;  // this thread's slot: 2 float4 per checkpoint
-  __device__ __forceinline__ void store(int j, const float (&m)[8]) const {
-    base[2 * j] = make_float4(m[0], m[1], m[2], m[3]);
-    base[2 * j + 1] = make_float4(m[4], m[5], m[6], m[7]);
-  }
-  __device__ __forceinline__ void load(int j, float (&m)[8]) const {
-    const float4 x = base[2 * j], y = base[2 * j + 1];
-    m[0] = x.x; m[1] = x.y; m[2] = x.z; m[3] = x.w; m[4] = y.x; m[5] = y.y; m[6] = y.z; m[7] = y.w;
-  }
-};
-
-// Global scratch with the windows of a launch interleaved: checkpoint plane j holds one float4
+// Checkpoint storage, 8 floats per checkpoint as two float4, in global scratch with the windows of
+// a launch interleaved: checkpoint plane j holds one float4
 // pair per window, so the 32 lanes of a warp (consecutive windows) store and load 32
 // consecutive float4 -- four whole cache lines -- per instruction.
 struct CkptStrided {
@@ -179,25 +126,54 @@ __device__ __forceinline__ void tail_llrs(bool lower, const float* d0, int k, fl
 
 constexpr float kDestMaxA = 1024.0f;
 
-// Runs window w of block cb for one half-iteration.  g = launch-wide window index (seed slot).
-// lower: the SISO over interleaved order; post (lower SISO only): also write the posterior
-// Ls + e1 + e2 (last iteration, early stop).  Both may be compile-time constants (the plain
-// kernels, one specialisation each) or run-time values (the persistent kernel, which keeps a
-// single copy of this code for both halves).  COHERENT: a-priori and seeds were written earlier
-// in the same kernel (persistent schedule).  TAPE: the alpha warm-up steps also leave
-// checkpoints, at negative indexes (q - lo) / S (the caller's checkpoint store is offset by the
-// warm-up), so that [a_lo, hi] is covered every S steps for the adjoint.
-template <int S, class Ckpt, bool COHERENT, bool STD = false, bool SMALL_LOOPS = false,
-          bool TAPE = false>
-__device__ __forceinline__ void siso_window_rt(const DevCb& cb, int w, int g, const SisoIo& io,
-                                               const Ckpt& ck, const bool LOWER, const bool POST) {
+// Where a window's inputs come from and its results go: the streams, seeds and outputs of a launch
+// in global memory (a launch per half-iteration).  g = launch-wide window index (seed slot).
+template <bool LOWER, bool POST, bool TAPE>
+struct GlobalAccess {
+  const SisoIo& io;
+  const DevCb& cb;
+  int g;
+  const float *d0, *sys, *par, *apr;
+  const uint16_t* pt;
+  __device__ __forceinline__ GlobalAccess(const SisoIo& io_, const DevCb& cb_, int g_)
+      : io(io_), cb(cb_), g(g_) {
+    d0 = io.llr + cb.llr;
+    sys = LOWER ? io.sys_i + cb.work : d0;
+    par = d0 + (LOWER ? 2 : 1) * (cb.k + 4);
+    apr = io.apr + cb.work;
+    pt = (LOWER ? io.perm : io.inv) + cb.tab;
+  }
+  __device__ __forceinline__ int guard() const { return io.guard; }
+  __device__ __forceinline__ float scale() const { return io.scale; }
+  __device__ __forceinline__ Raw4 raw4(int q) const { return load_raw4(sys, apr, par, q); }
+  __device__ __forceinline__ Raw8 raw8(int q) const { return load_raw8(sys, apr, par, q); }
+  // seeds: alpha of this window, beta of this window, alpha of the next, beta of the previous one
+  __device__ __forceinline__ void load_seed(bool beta, float (&v)[8]) const {
+    const float* p = io.seed_in + 16 * g + (beta ? 8 : 0);
+    const float4 x = ld4(p), y = ld4(p + 4);
+    v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
+  }
+  __device__ __forceinline__ void store_seed(bool beta, const float (&v)[8]) const {
+    float4* o = reinterpret_cast<float4*>(io.seed_out + (beta ? 16 * (g - 1) + 8 : 16 * (g + 1)));
+    o[0] = make_float4(v[0], v[1], v[2], v[3]);
+    o[1] = make_float4(v[4], v[5], v[6], v[7]);
+  }
+  // where the extrinsics of 4 steps go (4 x uint16), and one extrinsic there
+  __device__ __forceinline__ uint2 targets(int q) const { return __ldg(reinterpret_cast<const uint2*>(pt + q)); }
+  __device__ __forceinline__ void put(int q, int n, float e, float sa) const {
+    if (TAPE) io.tape[cb.work + q] = kLog2e * sa;
+    io.ext[cb.work + n] = e;
+    if (POST) io.post[cb.out + n] = sa + e;
+  }
+};
+
+// Runs window w of block cb for one half-iteration of the upper or (LOWER) the lower SISO, whose
+// inputs and outputs `io` reaches (GlobalAccess above; POST there: also the posterior).
+template <int S, bool LOWER, bool STD, class Access, class Ckpt>
+__device__ __forceinline__ void siso_window(const DevCb& cb, int w, const Access& io, const Ckpt& ck) {
   static_assert(S == 4, "sub-windows are one float4 group of 4 steps");
-  const int K = cb.k, W = cb.window, G = io.guard;
+  const int K = cb.k, W = cb.window, G = io.guard();
   const int lo = w * W, hi = min(lo + W, K);
-  const float* d0 = io.llr + cb.llr;
-  const float* sys = LOWER ? io.sys_i + cb.work : d0;
-  const float* par = d0 + (LOWER ? 2 : 1) * (K + 4);
-  const float* apr = io.apr + cb.work;
   const int nsub = (hi - lo) / S;
   float sa[4], a[4], b[4];
 
@@ -210,34 +186,16 @@ __device__ __forceinline__ void siso_window_rt(const DevCb& cb, int w, int g, co
     a_lo = 0;
     alpha_start(al);
   } else {
-    const float4 x = ld4_io<COHERENT>(io.seed_in + 16 * g), y = ld4_io<COHERENT>(io.seed_in + 16 * g + 4);
-    al[0] = x.x; al[1] = x.y; al[2] = x.z; al[3] = x.w; al[4] = y.x; al[5] = y.y; al[6] = y.z; al[7] = y.w;
+    io.load_seed(false, al);
   }
   float amax = 0.0f;  // largest |a| of the window (it covers [lo, hi))
-  if constexpr (SMALL_LOOPS) {  // 4-step groups; the next group is requested early
-    Raw4 cur = load_raw4<COHERENT>(sys, apr, par, a_lo);
-    for (int q = a_lo; q < hi; q += 4) {
-      Raw4 nxt = cur;
-      if (q + 4 < hi) nxt = load_raw4<COHERENT>(sys, apr, par, q + 4);
-      if (TAPE || q >= lo) {
-        float v[8];
-        ms_to_log(al, as, v);
-        ck.store((q - lo) / S, v);
-      }
-      scale4(cur, sa, a, b);
-      amax = fmaxf(amax, fmaxf(fmaxf(fabsf(a[0]), fabsf(a[1])), fmaxf(fabsf(a[2]), fabsf(a[3]))));
-#pragma unroll
-      for (int t = 0; t < 4; ++t) alpha_step_ms<STD>(al, as, a[t], b[t]);
-      ms_renorm(al, as);
-      cur = nxt;
-    }
-  } else {  // 8-step groups (both halves of each sector); the next group is requested early
-    Raw8 cur = load_raw8<COHERENT>(sys, apr, par, a_lo);
+  {  // 8-step groups (both halves of each sector); the next group is requested early
+    Raw8 cur = io.raw8(a_lo);
     for (int q = a_lo; q < hi; q += 8) {
       Raw8 nxt = cur;
-      if (q + 8 < hi) nxt = load_raw8<COHERENT>(sys, apr, par, q + 8);
+      if (q + 8 < hi) nxt = io.raw8(q + 8);
       float v[8];
-      if (TAPE || q >= lo) {
+      if (q >= lo) {
         ms_to_log(al, as, v);
         ck.store((q - lo) / S, v);
       }
@@ -245,7 +203,7 @@ __device__ __forceinline__ void siso_window_rt(const DevCb& cb, int w, int g, co
       amax = fmaxf(amax, fmaxf(fmaxf(fabsf(a[0]), fabsf(a[1])), fmaxf(fabsf(a[2]), fabsf(a[3]))));
 #pragma unroll
       for (int t = 0; t < 4; ++t) alpha_step_ms<STD>(al, as, a[t], b[t]);
-      if (TAPE || q >= lo) {
+      if (q >= lo) {
         ms_to_log(al, as, v);
         ck.store((q - lo) / S + 1, v);
       }
@@ -270,9 +228,7 @@ __device__ __forceinline__ void siso_window_rt(const DevCb& cb, int w, int g, co
     } else {
       ck.load((hi - G - lo) / S, r);
     }
-    float4* o = reinterpret_cast<float4*>(io.seed_out + 16 * (g + 1));
-    o[0] = make_float4(r[0], r[1], r[2], r[3]);
-    o[1] = make_float4(r[4], r[5], r[6], r[7]);
+    io.store_seed(false, r);
   }
 
   // ---- backward: warm-up from b_hi down to hi ----
@@ -282,29 +238,16 @@ __device__ __forceinline__ void siso_window_rt(const DevCb& cb, int w, int g, co
   if (b_hi >= K) {
     b_hi = K;
     float ts[3], tp[3];
-    tail_llrs<STD>(LOWER, d0, K, ts, tp);
+    tail_llrs<STD>(LOWER, io.d0, K, ts, tp);
     tail_beta<STD>(be, ts, tp);
   } else {
-    const float4 x = ld4_io<COHERENT>(io.seed_in + 16 * g + 8), y = ld4_io<COHERENT>(io.seed_in + 16 * g + 12);
-    be[0] = x.x; be[1] = x.y; be[2] = x.z; be[3] = x.w; be[4] = y.x; be[5] = y.y; be[6] = y.z; be[7] = y.w;
+    io.load_seed(true, be);
   }
-  if (SMALL_LOOPS && b_hi > hi) {
-    Raw4 cur = load_raw4<COHERENT>(sys, apr, par, b_hi - 4);
-    for (int q = b_hi - 4; q >= hi; q -= 4) {
-      Raw4 nxt = cur;
-      if (q - 4 >= hi) nxt = load_raw4<COHERENT>(sys, apr, par, q - 4);
-      scale4(cur, sa, a, b);
-#pragma unroll
-      for (int t = 3; t >= 0; --t) beta_step_ms<STD>(be, bs, a[t], b[t]);
-      ms_renorm(be, bs);
-      cur = nxt;
-    }
-  }
-  if (!SMALL_LOOPS && b_hi > hi) {
-    Raw8 cur = load_raw8<COHERENT>(sys, apr, par, b_hi - 8);
+  if (b_hi > hi) {
+    Raw8 cur = io.raw8(b_hi - 8);
     for (int q = b_hi - 8; q >= hi; q -= 8) {
       Raw8 nxt = cur;
-      if (q - 8 >= hi) nxt = load_raw8<COHERENT>(sys, apr, par, q - 8);
+      if (q - 8 >= hi) nxt = io.raw8(q - 8);
       scale4(cur.hi, sa, a, b);
 #pragma unroll
       for (int t = 3; t >= 0; --t) beta_step_ms<STD>(be, bs, a[t], b[t]);
@@ -316,12 +259,10 @@ __device__ __forceinline__ void siso_window_rt(const DevCb& cb, int w, int g, co
     }
   }
   const bool rec_beta = (w > 0) && (lo + G <= hi);
-  float4* bseed = rec_beta ? reinterpret_cast<float4*>(io.seed_out + 16 * (g - 1) + 8) : nullptr;
   if (rec_beta && lo + G == hi) {
     float r[8];
     ms_to_log(be, bs, r);
-    bseed[0] = make_float4(r[0], r[1], r[2], r[3]);
-    bseed[1] = make_float4(r[4], r[5], r[6], r[7]);
+    io.store_seed(true, r);
   }
 
   // ---- per 4-step sub-window (last to first): recompute alpha, then beta + extrinsic.  The
@@ -333,15 +274,14 @@ __device__ __forceinline__ void siso_window_rt(const DevCb& cb, int w, int g, co
   // The two are separate copies of the loop, each with its own register allocation. ----
   auto backward = [&](auto dest_tag) {
   constexpr bool DEST = decltype(dest_tag)::value && !STD;
-  const uint16_t* pt = (LOWER ? io.perm : io.inv) + cb.tab;
   Raw4 r_n;
   uint2 i_n;
   float c_n[8];
   float an[8];  // reference code: alpha at base + S (log values), the last step's alpha_{t+1}
   if (nsub > 0) {
     const int base = lo + (nsub - 1) * S;
-    r_n = load_raw4<COHERENT>(sys, apr, par, base);
-    i_n = __ldg(reinterpret_cast<const uint2*>(pt + base));
+    r_n = io.raw4(base);
+    i_n = io.targets(base);
     ck.load(nsub - 1, c_n);
     if constexpr (DEST) ck.load(nsub, an);
   }
@@ -357,8 +297,8 @@ __device__ __forceinline__ void siso_window_rt(const DevCb& cb, int w, int g, co
       As[0][k] = 1.0f;
     }
     if (j > 0) {
-      r_n = load_raw4<COHERENT>(sys, apr, par, base - S);
-      i_n = __ldg(reinterpret_cast<const uint2*>(pt + base - S));
+      r_n = io.raw4(base - S);
+      i_n = io.targets(base - S);
       ck.load(j - 1, c_n);
     }
     float SA[S], A_[S], B_[S];
@@ -375,16 +315,14 @@ __device__ __forceinline__ void siso_window_rt(const DevCb& cb, int w, int g, co
     const uint32_t w2[2] = {iv.x, iv.y};
     // step t's outputs, then beta_t
     auto finish = [&](int t, float e2) {
-      const float e = io.scale * (kLn2 * e2);
+      const float e = io.scale() * (kLn2 * e2);
       const int n = static_cast<int>((w2[t >> 1] >> (16 * (t & 1))) & 0xffffu);
-      io.ext[cb.work + n] = e;
-      if (POST) io.post[cb.out + n] = SA[t] + e;
+      io.put(base + t, n, e, SA[t]);
       beta_step_ms<STD>(be, bs, A_[t], B_[t]);
       if (rec_beta && base + t == lo + G) {
         float rr[8];
         ms_to_log(be, bs, rr);
-        bseed[0] = make_float4(rr[0], rr[1], rr[2], rr[3]);
-        bseed[1] = make_float4(rr[4], rr[5], rr[6], rr[7]);
+        io.store_seed(true, rr);
       }
     };
     if constexpr (DEST) {  // posterior from alpha_{t+1} beta_{t+1} minus Ls + La
@@ -407,13 +345,6 @@ __device__ __forceinline__ void siso_window_rt(const DevCb& cb, int w, int g, co
     backward(std::true_type{});
   else
     backward(std::false_type{});
-}
-
-template <int S, bool LOWER, bool POST, class Ckpt, bool COHERENT = false, bool STD = false,
-          bool TAPE = false>
-__device__ __forceinline__ void siso_window(const DevCb& cb, int w, int g, const SisoIo& io,
-                                            const Ckpt& ck) {
-  siso_window_rt<S, Ckpt, COHERENT, STD, false, TAPE>(cb, w, g, io, ck, LOWER, POST);
 }
 
 }  // namespace tcb
