@@ -50,3 +50,30 @@ def test_rate_matcher(tc, decoder, rv):
         assert np.array_equal(out[lo:lo + e], tc.rate_match(k, f, host[pos:pos + 3 * (k + 4)], e, r)), (k, f, e)
         lo += e
         pos += 3 * (k + 4)
+
+
+@pytest.mark.parametrize("form", ["tuples", "array", "floats"])
+def test_combining_takes_any_number_type(tc, decoder, form):
+    """Soft combining's descriptors as tuples of int, rows of an integer array, or floats."""
+    import torch
+
+    rng = np.random.default_rng(5)
+    tx, eo, lo = [], 0, 0
+    for k in (40, 1056):
+        for rv in range(3):
+            tx.append((k, 8, 2 * k, rv, eo, lo))
+            eo += 2 * k
+        lo += 3 * (k + 4)
+    e = torch.from_numpy(rng.normal(size=eo).astype(np.float32)).cuda()
+    ref = np.zeros(lo)
+    for k, f, n, rv, at, out in tx:
+        one = torch.zeros(lo, device="cuda")
+        decoder.derate_combine_device([(k, f, n, rv, at, 0)], e.data_ptr(), eo, one.data_ptr(), 3 * (k + 4))
+        torch.cuda.synchronize()
+        ref[out:out + 3 * (k + 4)] += one.cpu().numpy()[:3 * (k + 4)]
+    given = {"tuples": tx, "array": np.array(tx), "floats": [tuple(float(v) for v in t) for t in tx]}[form]
+    got = torch.zeros(lo, device="cuda")
+    decoder.derate_combine_device(given, e.data_ptr(), eo, got.data_ptr(), lo)
+    torch.cuda.synchronize()
+    # three sums of float32 values of size 1 to 5, in another order: 3 roundings of 2^-24 x 15
+    assert np.abs(got.cpu().numpy() - ref).max() <= 3e-6

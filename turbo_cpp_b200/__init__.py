@@ -9,7 +9,9 @@ from __future__ import annotations
 
 import ctypes as C
 import enum
+import itertools
 import os
+import struct
 from dataclasses import dataclass, field
 from typing import Optional, Sequence
 
@@ -88,6 +90,8 @@ class _RmBlock(C.Structure):
     _fields_ = [("k", C.c_int32), ("filler", C.c_int32), ("e", C.c_int32), ("rv", C.c_uint32),
                 ("e_offset", C.c_int64), ("llr_offset", C.c_int64)]
 
+
+_RM_BLOCK_STRUCT = struct.Struct("@iiiIqq")  # the same layout
 
 # numpy views of the descriptor structs (same field order, sizes and alignment)
 _CODE_BLOCK_DTYPE = np.dtype([("k", np.int32), ("filler", np.int32), ("llr_offset", np.int64),
@@ -644,10 +648,14 @@ class Decoder:
         """HARQ soft combining on the GPU: transmissions = (k, filler, e, rv, e_offset,
         llr_offset) tuples, those of one code block consecutive with the same llr_offset; each
         code block's [d0|d1|d2] becomes the sum of its transmissions' de-rate-matched LLRs."""
-        arr = (_RmBlock * max(len(transmissions), 1))()
-        for i, (k, f, e, rv, eo, lo) in enumerate(transmissions):
-            arr[i].k, arr[i].filler, arr[i].e, arr[i].rv = int(k), int(f), int(e), int(rv)
-            arr[i].e_offset, arr[i].llr_offset = int(eo), int(lo)
+        n = len(transmissions)
+        try:  # integers, as they mostly are: 0.16 ms for 2048 of them, attribute by attribute 1.6 ms
+            arr = (_RmBlock * n).from_buffer_copy(b"".join(itertools.starmap(_RM_BLOCK_STRUCT.pack, transmissions)))
+        except (struct.error, TypeError):  # anything int() takes
+            arr = (_RmBlock * max(n, 1))()
+            for i, (k, f, e, rv, eo, lo) in enumerate(transmissions):
+                arr[i].k, arr[i].filler, arr[i].e, arr[i].rv = int(k), int(f), int(e), int(rv)
+                arr[i].e_offset, arr[i].llr_offset = int(eo), int(lo)
         _call("tc_derate_combine_llr_device", self._h, len(transmissions), C.addressof(arr),
               int(e_len), e_ptr, int(llr_len), out_ptr, stream or None)
 
