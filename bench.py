@@ -14,7 +14,7 @@ Lines printed by rank 0 (one JSON object):
   e2e       -- the same metric through the C ABI with pinned host buffers: H2D of the LLRs,
                decode, D2H of posterior/flags inside the timed region (back-to-back
                tc_decode calls with TC_MEM_HOST_ASYNC; e2e.synchronous: TC_MEM_HOST calls)
-  roofline  -- dominant kernel (SISO half-iteration) against the SFU (MUFU) issue roofline
+  roofline  -- dominant kernel (SISO half-iteration) against the FP32 issue rate
   roofline_hbm -- the same kernel's algorithmic bytes against measured HBM bandwidth
   cpu_baseline -- the reference CPU decoder (oracle/_ref) on all host cores, bounded sample
   ber_bler  -- BER/BLER per Eb/N0 point of the GPU decode (and of the CPU sample)
@@ -39,11 +39,10 @@ sys.path.insert(0, ROOT)
 METRIC = "info Mbit/s @8 iters, matched BLER: batched vs plain GPU vs CPU ref; adjoint err"
 EBN0 = [0.0, 0.2, 0.4, 0.6, 0.8, 1.0, 1.2]
 K = 6144
-# algorithmic work of one trellis step of one SISO: 30 max*, 2 transcendentals each
-TRANSC_PER_STEP = 60
+FP32_PER_STEP = 40  # per trellis step of one SISO: alpha 16, beta 16, extrinsic 8
 # algorithmic HBM bytes per info bit of a whole decode: 3(K+4) LLRs in + K posteriors out
 BYTES_PER_BIT = 4.0 * (3 * (K + 4) + K) / K
-MUFU_PER_SM_CLK = 16  # B200 SFU lanes per SM per clock (4 per SM sub-partition)
+FP32_PER_SM_CLK = 128
 
 
 def parse():
@@ -766,16 +765,14 @@ def main():
     sm_mhz = clocks["sm_mhz"] or 1965.0
     avg_launch_ms = tm["siso_ms"] / max(tm["siso_launches"], 1)
     steps_per_launch = tm["trellis_steps"] / max(tm["siso_launches"], 1)
-    achieved = TRANSC_PER_STEP * steps_per_launch / (avg_launch_ms / 1e3) / 1e9
-    peak = props.multi_processor_count * MUFU_PER_SM_CLK * sm_mhz * 1e6 / 1e9
+    achieved = FP32_PER_STEP * steps_per_launch / (avg_launch_ms / 1e3) / 1e9
+    peak = props.multi_processor_count * FP32_PER_SM_CLK * sm_mhz * 1e6 / 1e9
     traffic_per_step = ncu_traffic(schedule_name)
     hbm_peak, hbm_src = measured_peaks()
     # algorithmic bytes of the launch: its share of the decode's 16 B per info bit
     alg_bytes_launch = steps_per_launch * BYTES_PER_BIT / (2 * it)
     hbm_achieved = alg_bytes_launch / (avg_launch_ms / 1e3) / 1e9
-    kernel_name = ("persistent_kernel (all iterations of all code blocks, device work queue)"
-                   if schedule_name == "persistent"
-                   else "siso_plain_kernel (one SISO half-iteration over all code blocks)")
+    kernel_name = "resident_kernel (all iterations of all code blocks, a CTA per task of blocks)"
     line = {
         "metric": METRIC, "value": value, "unit": "Mbit/s", "n_gpus": world,
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms / args.steps,
@@ -786,23 +783,20 @@ def main():
                      "guard": 96 if args.guard < 0 else args.guard,
                      "autotuned": tuned is not None, "cuda_graph": not args.no_graph},
         "roofline": {
-            "bound": "sfu", "achieved": achieved, "peak": peak, "unit": "Gtransc/s",
+            "bound": "fp32", "achieved": achieved, "peak": peak, "unit": "Gop/s",
             "frac": achieved / peak, "traffic": None if traffic_per_step is None
             else traffic_per_step * steps_per_launch,
             "kernel": kernel_name,
-            "work": f"{TRANSC_PER_STEP} transcendentals per trellis step per SISO (30 exact "
-                    f"max*), {steps_per_launch:.0f} SISO steps per launch",
+            "work": f"{FP32_PER_STEP} multiply-adds and multiplications per trellis step per SISO "
+                    f"(alpha 16, beta 16, extrinsic 8), {steps_per_launch:.0f} SISO steps per launch",
             "avg_launch_ms": avg_launch_ms,
-            "peak_source": f"{props.multi_processor_count} SMs x {MUFU_PER_SM_CLK} MUFU/clk x "
+            "peak_source": f"{props.multi_processor_count} SMs x {FP32_PER_SM_CLK} FP32/clk x "
                            f"median sampled SM clock {sm_mhz:.0f} MHz (nominal issue rate)",
-            "note": "achieved counts the reference formulation's work, 60 transcendentals per "
-                    "trellis step (30 exact max*, each an exp and a log1p), against the MUFU "
-                    "issue rate; the kernel's deferred-log arithmetic executes about 43 MUFU ops "
-                    "per output step (one ex2 per max* in the recursions, two 4-way log-sums for "
-                    "the extrinsic), so what binds is instruction issue (ncu: issue 69 % busy, "
-                    "XU 53 %, ~460 instructions per output step; "
-                    "profiles/siso_plain_kernel_k6144x4096.md); no tensor cores (not a "
-                    "contraction); HBM well below its peak (roofline_hbm)",
+            "note": "achieved counts the recursions' own arithmetic once; with the windows' warm-ups, the "
+                    "recomputed alpha, branch weights and checks the kernel executes about 160 "
+                    "instructions per step, 94 on the FMA pipe, and instruction issue binds "
+                    "(profiles/resident_kernel_k6144x1036.md); no tensor cores (not a contraction); HBM "
+                    "well below its peak (roofline_hbm)",
         },
         "roofline_hbm": {
             "bound": "hbm", "achieved": hbm_achieved, "peak": hbm_peak, "unit": "GB/s",
@@ -812,7 +806,7 @@ def main():
             else traffic_per_step * steps_per_launch / (avg_launch_ms / 1e3) / 1e9,
             "work": "16.0 B per info bit per decode (3(K+4) LLRs in, K posteriors out), the "
                     "launch's share; dram_gbs = the ncu DRAM bytes of a launch over its "
-                    "CUDA-event time (the working set streams from DRAM every half-iteration)",
+                    "CUDA-event time (the scratch slots of the resident CTAs are larger than L2)",
         },
         "gpu_launches": int(launches),
         "clocks": clocks,

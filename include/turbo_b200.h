@@ -191,8 +191,8 @@ TC_API int tc_autotune_load(tc_decoder* dec, const char* path);
 TC_API int tc_decoder_sync(tc_decoder* dec);
 
 /* Testing hook for the failure path (new): while set, persistent decodes on this decoder make
- * the warps working on task `task` (the task queue's order: largest blocks first) wait for a
- * progress count that is never reached.  The device-side wait limit (one second) runs out, the
+ * the CTA working on task `task` (the task queue's order: largest blocks first) wait for a word
+ * that is never written.  The device-side wait limit (one second) runs out, the
  * kernel still finishes, and the call reports TC_ERR_TIMEOUT (host memory) or tc_decoder_sync
  * does (device memory); the results of that call are not valid.  -1 turns it off. */
 TC_API int tc_decoder_inject_stall(tc_decoder* dec, int task);

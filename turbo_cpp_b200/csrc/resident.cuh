@@ -20,8 +20,8 @@
 //
 // The linear pass keeps all LLRs in base-2 units (natural LLR * log2(e)).
 //
-// What bounds it: the issue slots of the SMs (158 instructions per step of a half-iteration, warm-ups
-// included, 84 of them multiply-adds; the (m, s) form has about 450), at 2 warps per scheduler.  One warp
+// What bounds it: the issue slots of the SMs (161 instructions per step of a half-iteration, warm-ups
+// included, 84 of them multiplications and multiply-adds; the (m, s) form has about 450), at 2 warps per scheduler.  One warp
 // of 32 windows of 192 steps per CTA, because the shared memory of an SM holds X of 8 of them: 4096
 // blocks of K = 6144, 8 iterations: 2.83 ms with 8 CTAs per SM, 2.94 ms with 7 (rows of 33 words and a
 // ring of 4 stages), 8.5 ms with the (m, s) kernel that this one replaced.  One block of K = 6144 from
