@@ -1,7 +1,11 @@
 // adjoint.cu -- the hand-written adjoint of the unrolled, scaled Log-MAP iterations.
 //
-// Forward (taped): the decoder itself, which leaves in the tape what every half-iteration read: the
-// LLRs Ls + La in base-2 units and the SISO's order, and the seeds (Tape, decoder.hpp).
+// Forward (taped): the plain decoder's SISO kernel, one launch per half-iteration, with the
+// a-priori input and extrinsic output of every half-iteration kept in its own tape slot (slot j
+// is SISO j's a-priori, slot j+1 its scaled extrinsic; slot 0 is zero), the seeds of every
+// half-iteration in their own slab (SISO j reads slab j and writes slab j+2), and the alpha
+// checkpoints of every half-iteration in their own slab: every 4 steps from the window's alpha
+// start (seed or block start) to its end, as log values.
 //
 // Backward: per half-iteration, last to first, one thread per window of the forward schedule
 // runs the adjoint of its window in two phases (base-2 metrics, as the forward):
@@ -164,12 +168,13 @@ __device__ __forceinline__ float dest_weights(const float (&ma)[8], const float 
 
 struct AdjIo {
   const float* llr;       // channel LLRs, [d0|d1|d2] per block
-  const float* s;         // the taped log2(e) (Ls + La) of this SISO (work layout, its order)
+  const float* sys_i;     // interleaved systematic LLRs (work layout)
+  const float* apr;       // the a-priori this SISO read in the forward pass (work layout)
   const float* ge;        // d loss / d (scaled extrinsic of this SISO), work layout, this SISO's
                           // order (the lower SISO's: interleaved)
   const float* seeds;     // [launch window][16]: the seeds this SISO used
-  float4* alpha_ckpt;     // alpha checkpoints: ckpt_slots planes of n_win float4 pairs, plane m =
-                          // alpha at a_lo + 4m
+  float4* alpha_ckpt;     // the taped alpha checkpoints of this SISO: ckpt_slots planes of n_win
+                          // float4 pairs, plane m = alpha at a_lo + 4m
   float* own_sa;          // [work]: d loss / d(Ls+La) of the window's own steps (SISO order),
                           // phase 1's part; phase 2's part follows at own_sa + 2 * work
   float* own_par;         // [work]: d loss / d Lp (likewise)
@@ -186,13 +191,6 @@ struct AdjIo {
 __device__ __forceinline__ void load8(const float* p, float (&m)[8]) {
   const float4 x = ld4(p), y = ld4(p + 4);
   m[0] = x.x; m[1] = x.y; m[2] = x.z; m[3] = x.w; m[4] = y.x; m[5] = y.y; m[6] = y.z; m[7] = y.w;
-}
-
-// a = (log2(e) / 2) (Ls + La) and b = (log2(e) / 2) Lp of 4 consecutive steps
-__device__ __forceinline__ void load_steps(const float* s2, const float* par, int q, float (&a)[4], float (&b)[4]) {
-  const float4 x = ld4(s2 + q), y = ld4(par + q);
-  a[0] = 0.5f * x.x; a[1] = 0.5f * x.y; a[2] = 0.5f * x.z; a[3] = 0.5f * x.w;
-  b[0] = kHalfLog2e * y.x; b[1] = kHalfLog2e * y.y; b[2] = kHalfLog2e * y.z; b[3] = kHalfLog2e * y.w;
 }
 
 // d loss / d e of 4 consecutive positions of this SISO
@@ -220,35 +218,18 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjMinBlocks) siso_adjoint_kerne
   if (start) a_lo = 0;
   if (tail) b_hi = K;
   const float* d0 = io.llr + cb.llr;
+  const float* sys = LOWER ? io.sys_i + cb.work : d0;
   const float* par = d0 + (LOWER ? 2 : 1) * (K + 4);
-  const float* s2 = io.s + cb.work;
-  // alpha and beta checkpoints, each a slab of planes with the launch's windows
+  const float* apr = io.apr + cb.work;
+  // alpha (taped) and beta checkpoints, each a slab of planes with the launch's windows
   // interleaved
   const CkptStrided cka{io.alpha_ckpt, n_win, g};
   const CkptStrided ckb{io.ckpt, n_win, g};
-  float a[4], b[4];
+  float sa[4], a[4], b[4];
   float* ag = io.guard_g + static_cast<int64_t>(4 * g) * G;
   const float xs = kLn2 * io.scale;  // d e / d(base-2 extrinsic)
 
   if (PHASES & 1) {
-  {  // alpha from the seed or the block start, a checkpoint (log values) every 4 steps
-    float al[8], as[8];
-    ms_ones(as);
-    if (start) alpha_start(al);
-    else load8(io.seeds + 16 * g, al);
-    for (int q = a_lo; q < hi; q += 4) {
-      float v[8];
-      ms_to_log(al, as, v);
-      cka.store((q - a_lo) >> 2, v);
-      load_steps(s2, par, q, a, b);
-#pragma unroll
-      for (int t = 0; t < 4; ++t) alpha_step_ms<STD>(al, as, a[t], b[t]);
-      ms_renorm(al, as);
-    }
-    float v[8];
-    ms_to_log(al, as, v);
-    cka.store((hi - a_lo) >> 2, v);
-  }
   // ---- phase 1: backward in time ----
   float be[8];
   if (tail) {
@@ -265,7 +246,7 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjMinBlocks) siso_adjoint_kerne
       float v[8];
       ms_to_log(be, bs, v);
       ckb.store((P - lo) >> 2, v);
-      load_steps(s2, par, P - 4, a, b);
+      scale4(load_raw4(sys, apr, par, P - 4), sa, a, b);
 #pragma unroll
       for (int t = 3; t >= 0; --t) beta_step_ms<STD>(be, bs, a[t], b[t]);
       ms_renorm(be, bs);
@@ -285,7 +266,7 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjMinBlocks) siso_adjoint_kerne
   for (int P = hi; P > lo; P -= 4) {  // the window's own steps
     ckb.store((P - lo) >> 2, be);
     const int q = P - 4;
-    load_steps(s2, par, q, a, b);
+    scale4(load_raw4(sys, apr, par, q), sa, a, b);
     float ge[4];
     load_ge(io, cb, q, ge);
     float Al[4][8];
@@ -337,7 +318,7 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjMinBlocks) siso_adjoint_kerne
   }
   for (int P = lo; P > a_lo; P -= 4) {  // alpha warm-up steps
     const int q = P - 4;
-    load_steps(s2, par, q, a, b);
+    scale4(load_raw4(sys, apr, par, q), sa, a, b);
     float Al[4][8];
     cka.load((q - a_lo) >> 2, Al[0]);
 #pragma unroll
@@ -374,7 +355,7 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjMinBlocks) siso_adjoint_kerne
   cka.load((lo - a_lo) >> 2, al);
   float* bg = ag + 2 * G;
   for (int P = lo; P < b_hi; P += 4) {
-    load_steps(s2, par, P, a, b);
+    scale4(load_raw4(sys, apr, par, P), sa, a, b);
     float Bt[4][8];  // Bt[t] = beta at P + t + 1
     ckb.load((P + 4 - lo) >> 2, Bt[3]);
 #pragma unroll
@@ -680,7 +661,7 @@ T* reserve(DeviceBuffer& b, size_t count) {
 }  // namespace
 
 Adjoint::~Adjoint() {
-  for (DeviceBuffer* b : {&d_cbs_, &d_wincb_, &d_tape_, &d_seeds_, &d_ackpt_, &d_ckpt_,
+  for (DeviceBuffer* b : {&d_cbs_, &d_wincb_, &d_sysi_, &d_tape_, &d_seeds_, &d_tapeckpt_, &d_ckpt_,
                           &d_own_, &d_guard_, &d_tail_, &d_part_, &d_cbpart_, &d_ge2_, &d_ga1_})
     b->release();
 }
@@ -745,27 +726,47 @@ uint64_t Adjoint::forward(const AdjointRequest& rq) {
 
   DevCb* dcbs = reserve<DevCb>(d_cbs_, n);
   int32_t* dwin = reserve<int32_t>(d_wincb_, n_win);
-  float* tape = reserve<float>(d_tape_, 2 * static_cast<size_t>(I) * work);
+  float* sysi = reserve<float>(d_sysi_, work);
+  float* tape = reserve<float>(d_tape_, static_cast<size_t>(2 * I + 1) * work);
   const size_t slab = static_cast<size_t>(n_win) * 16;
-  float* seeds = reserve<float>(d_seeds_, (2 * static_cast<size_t>(I) + 2) * slab);
+  float* seeds = reserve<float>(d_seeds_, (2 * I + 2) * slab);
+  // alpha checkpoints of every half-iteration, a slab each
+  const size_t aslab = ckpt_slab(n_win, 2 * static_cast<size_t>(ckpt_bwd_));
+  float4* actp = reserve<float4>(d_tapeckpt_, 2 * I * aslab);
   ok(cudaMemcpyAsync(dcbs, cbs_.data(), n * sizeof(DevCb), cudaMemcpyHostToDevice, st), "copy descriptors");
   ok(cudaMemcpyAsync(dwin, wincb.data(), n_win * sizeof(int32_t), cudaMemcpyHostToDevice, st), "copy descriptors");
   ok(cudaMemsetAsync(seeds, 0, 2 * slab * sizeof(float), st), "zero seeds");
-  DecodeRequest d;
-  d.n_cb = n;
-  d.cbs = rq.cbs;
-  d.llr_len = rq.llr_len;
-  d.llr = rq.llr;
-  d.post_len = rq.post_len;
-  d.posterior = rq.posterior;
-  d.max_iterations = I;
-  d.window = window_req;
-  d.guard = guard;
-  d.device_memory = true;
-  d.scales = scales_.data();
-  d.std3gpp = rq.std3gpp;
-  d.stream = rq.stream;
-  launches_ += dec_.decode_taped(d, Tape{dcbs, tape, work, seeds, static_cast<int64_t>(slab)});
+  const uint16_t* dperm = dec_.perm_table();
+  const uint16_t* dinv = dec_.inv_table();
+  // sys_i and tape slot 0 (the first a-priori, zero)
+  launch_setup(dcbs, static_cast<int>(n), rq.llr, dperm, sysi, tape, st);
+  ok(cudaGetLastError(), "setup launch");
+  launches_ += 1;
+  const int blocks = (n_win + kThreads - 1) / kThreads;
+  for (uint32_t j = 0; j < 2 * I; ++j) {
+    const bool lower = j & 1;
+    SisoIo io{rq.llr, sysi, tape + j * work, tape + (j + 1) * work,
+              (j + 1 == 2 * I) ? rq.posterior : nullptr, dperm, dinv, seeds + j * slab,
+              seeds + (j + 2) * slab, scales_[j], guard};
+    float4* ck = actp + j * aslab;
+    if (rq.std3gpp) {
+      if (!lower)
+        siso_plain_kernel<kSub, 0, true, true><<<blocks, kThreads, 0, st>>>(dcbs, dwin, n_win, io, nullptr, ck);
+      else if (j + 1 < 2 * I)
+        siso_plain_kernel<kSub, 1, true, true><<<blocks, kThreads, 0, st>>>(dcbs, dwin, n_win, io, nullptr, ck);
+      else
+        siso_plain_kernel<kSub, 2, true, true><<<blocks, kThreads, 0, st>>>(dcbs, dwin, n_win, io, nullptr, ck);
+    } else {
+      if (!lower)
+        siso_plain_kernel<kSub, 0, false, true><<<blocks, kThreads, 0, st>>>(dcbs, dwin, n_win, io, nullptr, ck);
+      else if (j + 1 < 2 * I)
+        siso_plain_kernel<kSub, 1, false, true><<<blocks, kThreads, 0, st>>>(dcbs, dwin, n_win, io, nullptr, ck);
+      else
+        siso_plain_kernel<kSub, 2, false, true><<<blocks, kThreads, 0, st>>>(dcbs, dwin, n_win, io, nullptr, ck);
+    }
+    ok(cudaGetLastError(), "SISO launch");
+    launches_ += 1;
+  }
   have_tape_ = true;
   return ++tape_id_;
 }
@@ -791,9 +792,11 @@ void Adjoint::backward(uint64_t tape_id, const float* grad_post, float* grad_llr
   float* ge2 = reserve<float>(d_ge2_, work);
   float* ga1 = reserve<float>(d_ga1_, work);
   float4* ckpt = reserve<float4>(d_ckpt_, ckpt_slab(n_win, 2 * static_cast<size_t>(ckpt_bwd_)));
-  float4* ackpt = reserve<float4>(d_ackpt_, ckpt_slab(n_win, 2 * static_cast<size_t>(ckpt_bwd_)));
+  const size_t aslab = ckpt_slab(n_win, 2 * static_cast<size_t>(ckpt_bwd_));
+  float4* actp = static_cast<float4*>(d_tapeckpt_.ptr);
   const DevCb* dcbs = static_cast<const DevCb*>(d_cbs_.ptr);
   const int32_t* dwin = static_cast<const int32_t*>(d_wincb_.ptr);
+  const float* sysi = static_cast<const float*>(d_sysi_.ptr);
   const float* tape = static_cast<const float*>(d_tape_.ptr);
   const float* seeds = static_cast<const float*>(d_seeds_.ptr);
   const uint16_t* dperm = dec_.perm_table();
@@ -809,7 +812,8 @@ void Adjoint::backward(uint64_t tape_id, const float* grad_post, float* grad_llr
   for (int j = static_cast<int>(2 * I) - 1; j >= 0; --j) {
     const bool lower = j & 1;
     const bool last = j + 2 >= static_cast<int>(2 * I);  // a SISO of the last iteration
-    AdjIo io{llr_, tape + j * work, lower ? ge2 : ga1, seeds + j * slab, ackpt, own,
+    AdjIo io{llr_, sysi, tape + j * work, lower ? ge2 : ga1, seeds + j * slab,
+             actp + j * aslab, own,
              own + work, work, guard_g, tail_g, part, ckpt, ckpt_bwd_,
              scales_[j], G};
     if (std3gpp_) {

@@ -17,8 +17,9 @@ constexpr int kThreads = 64;  // threads (windows) per block of the plain SISO k
 constexpr int kMinBlocks = 8;  // 16 warps per SM: at most 128 registers per thread
 
 // KIND: 0 = upper SISO, 1 = lower SISO, 2 = lower SISO that also writes the posterior;
-// STD: the TS 36.212 code instead of the reference's; TAPE: a taped forward pass (SisoIo::tape).  The
-// checkpoint slab holds planes of n_win float4 pairs (windows interleaved).
+// STD: the TS 36.212 code instead of the reference's; TAPE: the alpha checkpoints cover
+// the warm-up too, plane (q - a_lo) / S of the slab for step q, and stay for the adjoint (a slab of
+// (window + guard) / S + 1 planes).  The checkpoint slab holds planes of n_win float4 pairs (windows interleaved).
 template <int S, int KIND, bool STD = false, bool TAPE = false>
 __global__ void __launch_bounds__(kThreads, kMinBlocks) siso_plain_kernel(const DevCb* __restrict__ cbs,
                                                               const int32_t* __restrict__ win_cb,
@@ -31,8 +32,10 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) siso_plain_kernel(const 
   if (done != nullptr && done[c]) return;
   const DevCb cb = cbs[c];
   const int w = g - cb.win0;
-  const CkptStrided ck{ckpt, n_win, g};
-  siso_window<S, KIND != 0, STD>(cb, w, GlobalAccess<KIND != 0, KIND == 2, TAPE>(io, cb, g), ck);
+  CkptStrided ck{ckpt, n_win, g};
+  if (TAPE)  // plane 0 is alpha at a_lo
+    ck.p += static_cast<int64_t>(2 * (min(w * cb.window, io.guard) / S)) * n_win;
+  siso_window<S, KIND != 0, STD, TAPE>(cb, w, GlobalAccess<KIND != 0, KIND == 2>(io, cb, g), ck);
 }
 
 // sys_i[i] = d0[Pi(i)]; E2 = 0 (first a-priori).  One CTA per code block: d0 is read into shared

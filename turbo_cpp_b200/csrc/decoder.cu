@@ -583,14 +583,7 @@ void Decoder::check_request(const DecodeRequest& rq) const {
   }
 }
 
-uint64_t Decoder::decode_taped(const DecodeRequest& rq, const Tape& tape) {
-  std::lock_guard<std::mutex> lock(mu_);
-  const uint64_t before = timing_.launches;
-  decode_now(rq, &tape);
-  return timing_.launches - before;
-}
-
-void Decoder::decode_now(const DecodeRequest& rq, const Tape* tape) {
+void Decoder::decode_now(const DecodeRequest& rq) {
   check(cudaSetDevice(device_), "cudaSetDevice");
   // device memory: the caller's stream as given (NULL = legacy default stream, as in CUDA);
   // host memory: the caller's stream if given, else the decoder's own stream
@@ -648,9 +641,9 @@ void Decoder::decode_now(const DecodeRequest& rq, const Tape* tape) {
   }
   pack_tasks(rq, l);
   if (l.resident)
-    run_resident(rq, l, io, st, tape);
+    run_resident(rq, l, io, st);
   else
-    run_sweeps(rq, l, io, st, tape);
+    run_sweeps(rq, l, io, st);
   if (!rq.device_memory) {
     check(cudaMemcpyAsync(rq.posterior, io.post, rq.post_len * sizeof(float), cudaMemcpyDeviceToHost, st),
           "copy posterior out");
@@ -672,6 +665,12 @@ void Decoder::decode_now(const DecodeRequest& rq, const Tape* tape) {
 void Decoder::pack_tasks(const DecodeRequest& rq, Layout& l) const {
   const size_t n = l.cbs.size();
   if (rq.max_iterations > static_cast<uint32_t>(kMaxIterations) || l.max_windows > kResMaxThreads) return;
+  // Windows asked for below the default length are the differentiable decoder's (64 steps).  The gradient
+  // of its extrinsic scales is a sum whose terms cancel: the rounding of the forward pass alone moves it
+  // by 1 to 3e-5 of its norm.  Its forward pass keeps the (m, s) kernels (1024 x K = 6144, 6 iterations,
+  // forward and backward: 7.0 ms; 6.7 ms with this kernel as the forward pass), and so does the plain
+  // decode that has to equal it bit for bit.
+  if (!rq.persistent && rq.window > 0 && rq.window < kDefaultWindow) return;
   // threads per CTA: one warp when every block fits in it; else the multiple of 32 up to 128 that
   // whole blocks of the largest window count fill best (48 windows of K = 6144 at 128 steps: two
   // blocks in 96), unless the batch is too small to give every SM a CTA of several blocks
@@ -722,7 +721,7 @@ void Decoder::pack_tasks(const DecodeRequest& rq, Layout& l) const {
   l.resident = l.max_window <= 1024 || tasks <= per_sm * sm_count_;
 }
 
-void Decoder::run_resident(const DecodeRequest& rq, const Layout& l, const Io& io, void* stream, const Tape* tape) {
+void Decoder::run_resident(const DecodeRequest& rq, const Layout& l, const Io& io, void* stream) {
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const size_t n = l.res.size();
   const int tasks = static_cast<int>(l.task_first.size()) - 1;
@@ -763,7 +762,6 @@ void Decoder::run_resident(const DecodeRequest& rq, const Layout& l, const Io& i
   a.guard = l.guard;
   a.max_iterations = static_cast<int>(rq.max_iterations);
   a.early_stop = rq.early_stop ? 1 : 0;
-  if (tape != nullptr) a.tape = *tape;
   a.crc_ok = io.crc;
   a.iters = io.iters;
   record_start(st);
@@ -775,16 +773,16 @@ void Decoder::run_resident(const DecodeRequest& rq, const Layout& l, const Io& i
 
 namespace {
 // one SISO launch: kind 0 upper, 1 lower, 2 lower + posterior
-template <bool STD, bool TAPE>
+template <bool STD>
 void launch_siso(int kind, int blocks, cudaStream_t st, const DevCb* dcbs, const int32_t* dwin,
                  int n_win, const SisoIo& io, const uint8_t* dn, float4* ckpt) {
-  if (kind == 0) siso_plain_kernel<kSub, 0, STD, TAPE><<<blocks, kThreads, 0, st>>>(dcbs, dwin, n_win, io, dn, ckpt);
-  else if (kind == 1) siso_plain_kernel<kSub, 1, STD, TAPE><<<blocks, kThreads, 0, st>>>(dcbs, dwin, n_win, io, dn, ckpt);
-  else siso_plain_kernel<kSub, 2, STD, TAPE><<<blocks, kThreads, 0, st>>>(dcbs, dwin, n_win, io, dn, ckpt);
+  if (kind == 0) siso_plain_kernel<kSub, 0, STD><<<blocks, kThreads, 0, st>>>(dcbs, dwin, n_win, io, dn, ckpt);
+  else if (kind == 1) siso_plain_kernel<kSub, 1, STD><<<blocks, kThreads, 0, st>>>(dcbs, dwin, n_win, io, dn, ckpt);
+  else siso_plain_kernel<kSub, 2, STD><<<blocks, kThreads, 0, st>>>(dcbs, dwin, n_win, io, dn, ckpt);
 }
 }  // namespace
 
-void Decoder::run_sweeps(const DecodeRequest& rq, const Layout& l, const Io& io, void* stream, const Tape* tape) {
+void Decoder::run_sweeps(const DecodeRequest& rq, const Layout& l, const Io& io, void* stream) {
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const size_t n = l.cbs.size();
   std::vector<DevCb> cbs = l.cbs;
@@ -834,17 +832,10 @@ void Decoder::run_sweeps(const DecodeRequest& rq, const Layout& l, const Io& io,
     // the posterior is needed after the last iteration and, with early stop, after each one
     const bool post_now = rq.early_stop || it + 1 == rq.max_iterations;
     for (int half = 0; half < 2; ++half) {
-      SisoIo sio = half ? lo : up;
-      if (tape != nullptr) {
-        const int j = 2 * it + half;
-        sio.tape = tape->s + j * tape->stride;
-        sio.seed_in = tape->seeds + j * tape->slab;
-        sio.seed_out = tape->seeds + (j + 2) * tape->slab;
-      }
+      const SisoIo& sio = half ? lo : up;
       const int kind = half == 0 ? 0 : (post_now ? 2 : 1);
       record_start(st);
-      const auto launch = rq.std3gpp ? (tape ? launch_siso<true, true> : launch_siso<true, false>)
-                                     : (tape ? launch_siso<false, true> : launch_siso<false, false>);
+      const auto launch = rq.std3gpp ? launch_siso<true> : launch_siso<false>;
       launch(kind, blocks, st, dcbs, dwin, n_win, sio, dn, ckpt);
       check(cudaGetLastError(), "SISO launch");
       record_stop(st, static_cast<uint64_t>(l.steps));

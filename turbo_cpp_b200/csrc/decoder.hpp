@@ -49,19 +49,6 @@ struct CodeBlockDesc {
   int64_t out_offset;  // floats; K posterior LLRs
 };
 
-// Where a taped forward pass leaves what each half-iteration j reads: log2(e) (Ls + La) in the SISO's
-// order at s + j * stride + DevCb::work, the seeds (alpha, beta) of window DevCb::win0 + w at
-// seeds + j * slab + 16 (win0 + w).  Room for 2 slabs more: a launch per half-iteration writes the
-// seeds of j + 2; the first two are zero.
-struct DevCb;
-struct Tape {
-  const DevCb* cbs = nullptr;  // device; work and win0 of each block of the request, in its order
-  float* s = nullptr;
-  int64_t stride = 0;
-  float* seeds = nullptr;
-  int64_t slab = 0;
-};
-
 struct DecodeRequest {
   size_t n_cb = 0;
   const CodeBlockDesc* cbs = nullptr;  // host memory
@@ -147,9 +134,6 @@ class Decoder {
   Decoder(const Decoder&) = delete;
   Decoder& operator=(const Decoder&) = delete;
 
-  // A device-memory decode that also records the tape of its half-iterations (the differentiable
-  // decoder's forward pass); returns the kernels launched.
-  uint64_t decode_taped(const DecodeRequest& rq, const Tape& tape);
   void decode(const DecodeRequest& rq);  // plain or persistent schedule
   int device() const { return device_; }
   void set_timing(bool on);
@@ -197,13 +181,13 @@ class Decoder {
   // One decode: checks the request, cuts the blocks into windows (the two schedules differ in
   // the layout only) and runs the block-resident kernel, or, for layouts it cannot hold, one
   // launch per half-iteration.
-  void decode_now(const DecodeRequest& rq, const Tape* tape = nullptr);
+  void decode_now(const DecodeRequest& rq);
   struct Layout;  // windows of a request and their packing into tasks (decoder.cu)
   struct Io;      // device buffers of one call
   void check_request(const DecodeRequest& rq) const;
   void pack_tasks(const DecodeRequest& rq, Layout& l) const;
-  void run_resident(const DecodeRequest& rq, const Layout& l, const Io& io, void* stream, const Tape* tape);
-  void run_sweeps(const DecodeRequest& rq, const Layout& l, const Io& io, void* stream, const Tape* tape);
+  void run_resident(const DecodeRequest& rq, const Layout& l, const Io& io, void* stream);
+  void run_sweeps(const DecodeRequest& rq, const Layout& l, const Io& io, void* stream);
   // Asynchronous host-memory calls rotate over kAsyncWorkers worker decoders, each with its own
   // device buffers and stream: a call enqueues copy-in, decode and copy-out on the next worker
   // and returns, so that its copies run while the previous calls decode.  sync() waits for them.

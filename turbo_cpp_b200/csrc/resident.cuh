@@ -75,7 +75,6 @@ struct ResArgs {
   uint8_t* crc_ok;
   uint32_t* iters;
   const float* scale;         // [2 * max_iterations]
-  Tape tape;                  // of a taped forward pass (tape.s null: none)
 };
 
 __device__ __forceinline__ int load_acquire(const int* p) {
@@ -746,30 +745,6 @@ __device__ __noinline__ void put_extrinsics(const bool lower, const bool post) {
   }
 }
 
-// Taped forward pass: what a half-iteration of this thread's window reads, log2(e) (Ls + La) in the
-// SISO's order and the seeds.
-template <int NT>
-__device__ __noinline__ void res_tape(const Tape& t, const int cb, const int half, const float unit) {
-  const ResWin v = res_win<NT>();
-  const Slot<NT> m;
-  const bool lower = half & 1;
-  const char* const X = res_x<NT>();
-  const DevCb& d = t.cbs[cb];
-  float* o = t.s + half * t.stride + d.work + v.lo;
-#pragma unroll 2
-  for (int r = 0; r < v.len; r += 8, o += 8) {
-    const uint4 q = *reinterpret_cast<const uint4*>(m.base + m.record(lower, r >> 3) + m.kIndex + 16 * v.tid);
-    float s[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) s[k] = unit * lds(X, Ring<NT>::place(q, k));
-    *reinterpret_cast<float4*>(o) = make_float4(s[0], s[1], s[2], s[3]);
-    *reinterpret_cast<float4*>(o + 4) = make_float4(s[4], s[5], s[6], s[7]);
-  }
-  float4* const sd = reinterpret_cast<float4*>(t.seeds + half * t.slab + 16 * static_cast<int64_t>(d.win0 + v.w));
-#pragma unroll
-  for (int k = 0; k < 4; ++k) sd[k] = m.ld(m.seeds(lower, half >> 1) + k * m.kPlane + 16 * v.tid);
-}
-
 // X of this thread's window as the half-iteration that failed had it, in natural units.
 template <int NT>
 __device__ __noinline__ void res_restore(const bool lower) {
@@ -1054,7 +1029,7 @@ __device__ __noinline__ void log_half(const float* d0, const int it, const float
   cb.nwin = io.v.nwin;
   cb.window = io.v.window;
   const CkptStrided ck{reinterpret_cast<float4*>(io.m.base) + 12 * io.m.rows8 * NT, NT, io.v.tid};
-  siso_window<kSub, LOWER, STD>(cb, io.v.w, io, ck);
+  siso_window<kSub, LOWER, STD, false>(cb, io.v.w, io, ck);
 }
 
 template <bool STD, int NT>
@@ -1132,7 +1107,6 @@ __global__ void __launch_bounds__(NT, 256 / NT) resident_kernel(const __grid_con
         const bool lower = half & 1, last_half = half + 1 == 2 * p.max_iterations;
         const bool post_now = lower && (p.early_stop || last_half);
         const float scale = __ldg(p.scale + half);
-        if (p.tape.s != nullptr && run && half >= (pass == 0 ? 0 : from)) res_tape<NT>(p.tape, cb->idx, half, pass == 0 ? 1.0f : kLog2e);
         if (pass == 0) {
           // (a block that fails is left to the second pass)
           const bool keep = margin < kNear;

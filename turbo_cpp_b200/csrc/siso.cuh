@@ -47,7 +47,6 @@ struct SisoIo {
   float* seed_out;
   float scale;            // extrinsic scale of this half-iteration (1.0 for the plain decoder)
   int guard;
-  float* tape = nullptr;  // taped forward pass: log2(e) (Ls + La) in this SISO's order (work layout)
 };
 
 __device__ __forceinline__ float4 ld4(const float* p) {
@@ -128,7 +127,7 @@ constexpr float kDestMaxA = 1024.0f;
 
 // Where a window's inputs come from and its results go: the streams, seeds and outputs of a launch
 // in global memory (a launch per half-iteration).  g = launch-wide window index (seed slot).
-template <bool LOWER, bool POST, bool TAPE>
+template <bool LOWER, bool POST>
 struct GlobalAccess {
   const SisoIo& io;
   const DevCb& cb;
@@ -160,8 +159,7 @@ struct GlobalAccess {
   }
   // where the extrinsics of 4 steps go (4 x uint16), and one extrinsic there
   __device__ __forceinline__ uint2 targets(int q) const { return __ldg(reinterpret_cast<const uint2*>(pt + q)); }
-  __device__ __forceinline__ void put(int q, int n, float e, float sa) const {
-    if (TAPE) io.tape[cb.work + q] = kLog2e * sa;
+  __device__ __forceinline__ void put(int, int n, float e, float sa) const {
     io.ext[cb.work + n] = e;
     if (POST) io.post[cb.out + n] = sa + e;
   }
@@ -169,7 +167,9 @@ struct GlobalAccess {
 
 // Runs window w of block cb for one half-iteration of the upper or (LOWER) the lower SISO, whose
 // inputs and outputs `io` reaches (GlobalAccess above; POST there: also the posterior).
-template <int S, bool LOWER, bool STD, class Access, class Ckpt>
+// TAPE: the alpha warm-up steps also leave checkpoints, at negative indexes (q - lo) / S (the caller's
+// checkpoint store is offset by the warm-up), so that [a_lo, hi] is covered every S steps for the adjoint.
+template <int S, bool LOWER, bool STD, bool TAPE, class Access, class Ckpt>
 __device__ __forceinline__ void siso_window(const DevCb& cb, int w, const Access& io, const Ckpt& ck) {
   static_assert(S == 4, "sub-windows are one float4 group of 4 steps");
   const int K = cb.k, W = cb.window, G = io.guard();
@@ -195,7 +195,7 @@ __device__ __forceinline__ void siso_window(const DevCb& cb, int w, const Access
       Raw8 nxt = cur;
       if (q + 8 < hi) nxt = io.raw8(q + 8);
       float v[8];
-      if (q >= lo) {
+      if (TAPE || q >= lo) {
         ms_to_log(al, as, v);
         ck.store((q - lo) / S, v);
       }
@@ -203,7 +203,7 @@ __device__ __forceinline__ void siso_window(const DevCb& cb, int w, const Access
       amax = fmaxf(amax, fmaxf(fmaxf(fabsf(a[0]), fabsf(a[1])), fmaxf(fabsf(a[2]), fabsf(a[3]))));
 #pragma unroll
       for (int t = 0; t < 4; ++t) alpha_step_ms<STD>(al, as, a[t], b[t]);
-      if (q >= lo) {
+      if (TAPE || q >= lo) {
         ms_to_log(al, as, v);
         ck.store((q - lo) / S + 1, v);
       }
