@@ -3,7 +3,7 @@
 // One tc_decode call decodes any number of code blocks of any LTE sizes; every thread owns one
 // window of one code block.  The block-resident kernel (resident.cuh) runs all iterations in one
 // launch; layouts it cannot hold (very long windows in large batches, more than 256 windows per
-// block, more than 64 iterations) run as two launches per iteration (upper SISO over natural
+// block, more than 64 iterations) and the training schedule's short windows run as two launches per iteration (upper SISO over natural
 // order, lower SISO over QPP order) and, with early stop, one CRC24B launch.  This is the
 // replacement of the reference's Stage 1/2 host loops (lte_turbo_cuda.cu:1391-1540, 1719-1899),
 // batched over code blocks and correct for every K.

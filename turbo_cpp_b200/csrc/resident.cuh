@@ -20,12 +20,13 @@
 //
 // The linear pass keeps all LLRs in base-2 units (natural LLR * log2(e)).
 //
-// What bounds it: the issue slots of the SMs (161 instructions per step of a half-iteration, warm-ups
-// included, 84 of them multiplications and multiply-adds; the (m, s) form has about 450), at 2 warps per scheduler.  One warp
-// of 32 windows of 192 steps per CTA, because the shared memory of an SM holds X of 8 of them: 4096
-// blocks of K = 6144, 8 iterations: 2.83 ms with 8 CTAs per SM, 2.94 ms with 7 (rows of 33 words and a
-// ring of 4 stages), 8.5 ms with the (m, s) kernel that this one replaced.  One block of K = 6144 from
-// host memory: 0.44 ms (1.09 ms); 20000 mixed blocks with early stop: 6.8 ms (14.2 ms).
+// What bounds it: the issue slots of the SMs, at 2 warps per scheduler (161 instructions per step of a
+// half-iteration, warm-ups included, before most multiplications and multiply-adds went in pairs; the
+// (m, s) form has about 450).  One warp of 32 windows of 192 steps per CTA, because the shared memory of an
+// SM holds X of 8 of them (7 CTAs with rows of 33 words and a ring of 4 stages were 4 % slower).  4096
+// blocks of K = 6144, 8 iterations: 2.80 ms, 2.89 ms without the pairs, 8.0 ms with the (m, s) kernel that
+// this one replaced.  One block of K = 6144 from host memory: 0.43 ms (0.44, 1.08 ms); 20000 mixed blocks
+// with early stop: 6.2 ms (6.8, 14.3 ms).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -216,9 +217,96 @@ __device__ __forceinline__ void beta_std(const float (&be)[8], const float (&g)[
                   be[next_state<true>(s, 1)] * g[1][parity<true>(s, 1)]);
 }
 
-// One alpha step with weights w, one beta step with weights w scaled by r.
+// Packed pairs (fma.rn.f32x2 and mul.rn.f32x2: one issue slot for two operations, each rounded as the
+// scalar one, so that the results are bit for bit the same).  The reference code's recursions use them,
+// because issue slots are what the kernel runs out of: 4096 blocks of K = 6144 2892 -> 2800 us, 512 of them
+// with early stop 511 -> 488 us, 20000 mixed blocks 6797 -> 6167 us, 1000 of K = 1024 383 -> 355 us.  (In
+// lin_read alone: 2923 us where the whole takes 2728.)  The TS 36.212 code has 4 products of weights per
+// step that differ between the branches into a state, and stays scalar.
+__device__ __forceinline__ uint64_t pack2(float x, float y) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t p, float& x, float& y) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(p));
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+// The branches of the reference code with parity 0: the predecessor of state n, and its inverse.  The
+// branches with parity 1 come from unit_pred(n) ^ 1 and go to unit_succ(p) ^ 4.
+__host__ __device__ constexpr int unit_pred(int n) {
+  return (n >> 1 & 1) << 2 | (n & 1) << 1 | ((n >> 2 ^ n >> 1) & 1);
+}
+__host__ __device__ constexpr int unit_succ(int p) {
+  return ((p >> 2 ^ p) & 1) << 2 | (p >> 2 & 1) << 1 | (p >> 1 & 1);
+}
+// alpha_lin, beta_lin and input_scale on the pairs (s, s ^ M) of the states s without bit F; the results
+// are the pairs of unit_succ (alpha) or unit_pred (beta) of these.
+template <int M, int F>
+__device__ __forceinline__ void alpha_lin2(const float (&al)[8], float b, float (&at)[8]) {
+  const uint64_t bb = pack2(b, b);
+#pragma unroll
+  for (int s = 0; s < 8; ++s)
+    if ((s & F) == 0)
+      unpack2(fma2(bb, pack2(al[s ^ 1], al[s ^ 1 ^ M]), pack2(al[s], al[s ^ M])), at[unit_succ(s)],
+              at[unit_succ(s ^ M)]);
+}
+template <int M, int F>
+__device__ __forceinline__ void beta_lin2(const float (&bh)[8], float b, float (&be)[8]) {
+  const uint64_t bb = pack2(b, b);
+#pragma unroll
+  for (int s = 0; s < 8; ++s)
+    if ((s & F) == 0)
+      unpack2(fma2(bb, pack2(bh[s ^ 4], bh[s ^ 4 ^ M]), pack2(bh[s], bh[s ^ M])), be[unit_pred(s)],
+              be[unit_pred(s ^ M)]);
+}
+template <int M, int F>
+__device__ __forceinline__ void input_scale2(const float (&at)[8], float a1, float a0, float (&al)[8]) {
+#pragma unroll
+  for (int s = 0; s < 8; ++s)
+    if ((s & F) == 0)
+      unpack2(mul2(pack2(at[s], at[s ^ M]), pack2(pred_input<false>(s, 0) ? a1 : a0, pred_input<false>(s ^ M, 0) ? a1 : a0)),
+              al[s], al[s ^ M]);
+}
+
+// Step t of a group of 8.  The pairs of one step are the operands of the next one, in the same order of
+// their two states, for two steps; in the third the orders of the two operands differ (the map has no
+// functional that stays 0 on three parity branches), and the scalar step, which reads and leaves its
+// values in any register, brings back the first pairs.
+__device__ __forceinline__ void alpha_lin_at(int t, const float (&al)[8], float b, float (&at)[8]) {
+  if (t % 3 == 0) alpha_lin2<4, 4>(al, b, at);
+  else if (t % 3 == 1) alpha_lin2<6, 2>(al, b, at);
+  else alpha_lin(al, b, at);
+}
+__device__ __forceinline__ void alpha_scale_at(int t, const float (&at)[8], float a1, float a0, float (&al)[8]) {
+  if (t % 3 == 0) input_scale2<6, 2>(at, a1, a0, al);
+  else if (t % 3 == 1) input_scale2<7, 1>(at, a1, a0, al);
+  else input_scale2<4, 4>(at, a1, a0, al);
+}
+__device__ __forceinline__ void beta_at(int t, const float (&be)[8], const Weights& w, float (&out)[8]) {
+  float x[8];
+  const int phase = (7 - t) % 3;
+  if (t == 7) input_scale(be, w.a1, w.a0, x);  // the group before left other pairs
+  else if (phase == 0) input_scale2<1, 1>(be, w.a1, w.a0, x);
+  else if (phase == 1) input_scale2<2, 2>(be, w.a1, w.a0, x);
+  else input_scale2<5, 4>(be, w.a1, w.a0, x);
+  if (phase == 0) beta_lin2<1, 1>(x, w.b, out);
+  else if (phase == 1) beta_lin2<2, 2>(x, w.b, out);
+  else beta_lin(x, w.b, out);
+}
+
+// One alpha step with weights w, one beta step with weights w scaled by r: step t of a group.
 template <bool STD>
-__device__ __forceinline__ void alpha_next(float (&al)[8], const Weights& w) {
+__device__ __forceinline__ void alpha_next(int step, float (&al)[8], const Weights& w) {
   float t[8];
   if constexpr (STD) {
     float g[2][2];
@@ -227,12 +315,12 @@ __device__ __forceinline__ void alpha_next(float (&al)[8], const Weights& w) {
 #pragma unroll
     for (int n = 0; n < 8; ++n) al[n] = t[n];
   } else {
-    alpha_lin(al, w.b, t);
-    input_scale(t, w.a1, w.a0, al);
+    alpha_lin_at(step, al, w.b, t);
+    alpha_scale_at(step, t, w.a1, w.a0, al);
   }
 }
 template <bool STD>
-__device__ __forceinline__ void beta_next(float (&be)[8], Weights w, float r) {
+__device__ __forceinline__ void beta_next(int step, float (&be)[8], Weights w, float r) {
   w.a1 *= r;
   w.a0 *= r;
   float t[8];
@@ -243,8 +331,9 @@ __device__ __forceinline__ void beta_next(float (&be)[8], Weights w, float r) {
 #pragma unroll
     for (int n = 0; n < 8; ++n) be[n] = t[n];
   } else {
-    input_scale(be, w.a1, w.a0, t);
-    beta_lin(t, w.b, be);
+    beta_at(step, be, w, t);
+#pragma unroll
+    for (int n = 0; n < 8; ++n) be[n] = t[n];
   }
 }
 
@@ -496,13 +585,14 @@ __device__ __forceinline__ void lin_read(const ResWin& v, const Slot<NT>& m, con
 #pragma unroll
       for (int n = 0; n < 8; ++n) al[n] *= r;
       if (j >= 0) {
-        m.st8(ck, al);
+        const float o[8] = {al[0], al[4], al[1], al[5], al[2], al[6], al[3], al[7]};  // the pairs of step 0
+        m.st8(ck, o);
         ck += 2 * kPlane;
       }
       request(ring.at);
       ring.advance();
 #pragma unroll
-      for (int t = 0; t < 8; ++t) alpha_next<STD>(al, weights(s[t], b[t]));
+      for (int t = 0; t < 8; ++t) alpha_next<STD>(t, al, weights(s[t], b[t]));
     }
   }
   const int tail_at = v.k - (v.lo + v.len);  // steps of the block behind the window
@@ -512,7 +602,12 @@ __device__ __forceinline__ void lin_read(const ResWin& v, const Slot<NT>& m, con
   const bool seed_next = v.w + 1 < v.nwin;
   if (seed_next) {  // the next window's alpha seed: alpha at hi - guard
     float sd[8];
-    if (G > 0) m.ld8(m.ckpt((v.len - G) >> 3) + 16 * tid, al);
+    if (G > 0) {
+      float o[8];
+      m.ld8(m.ckpt((v.len - G) >> 3) + 16 * tid, o);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) al[(k >> 1) + 4 * (k & 1)] = o[k];
+    }
     log_from_lin(al, sd);
     m.st8(seed_out + 16 * v.next, sd);
   }
@@ -542,7 +637,7 @@ __device__ __forceinline__ void lin_read(const ResWin& v, const Slot<NT>& m, con
       ring.advance();
       const float r = rescale(be, v.top);
 #pragma unroll
-      for (int t = 7; t >= 0; --t) beta_next<STD>(be, weights(s[t], b[t]), t == 7 ? r : 1.0f);
+      for (int t = 7; t >= 0; --t) beta_next<STD>(t, be, weights(s[t], b[t]), t == 7 ? r : 1.0f);
     }
     if (tail_at == 0) {
 #pragma unroll
@@ -592,7 +687,8 @@ __device__ __forceinline__ float2 lin_write(const ResWin& v, const Slot<NT>& m, 
   for (; j >= 0; --j) {
     float s[8], b[8], a[8], base[8];
     const uint4 places = ring.read(X, s, b);
-    put(a, ca, cb);
+    a[0] = ca.x; a[4] = ca.y; a[1] = ca.z; a[5] = ca.w;  // (the order of the checkpoints)
+    a[2] = cb.x; a[6] = cb.y; a[3] = cb.z; a[7] = cb.w;
     put(base, la, lb);
     if (post) {
 #pragma unroll
@@ -624,10 +720,10 @@ __device__ __forceinline__ float2 lin_write(const ResWin& v, const Slot<NT>& m, 
       if constexpr (STD) {
 #pragma unroll
         for (int n = 0; n < 8; ++n) A[t][n] = a[n];
-        if (t < 7) alpha_next<STD>(a, wt[t]);
+        if (t < 7) alpha_next<STD>(t, a, wt[t]);
       } else {
-        alpha_lin(a, wt[t].b, A[t]);
-        if (t < 7) input_scale(A[t], wt[t].a1, wt[t].a0, a);
+        alpha_lin_at(t, a, wt[t].b, A[t]);
+        if (t < 7) alpha_scale_at(t, A[t], wt[t].a1, wt[t].a0, a);
       }
     }
     float e[8], xl = 0.0f;
@@ -667,7 +763,7 @@ __device__ __forceinline__ float2 lin_write(const ResWin& v, const Slot<NT>& m, 
       *reinterpret_cast<float*>(X + Ring<NT>::place(places, t)) = base[t] + e[t];
       if (keep_ext && (t & 3) == 0)
         *reinterpret_cast<float4*>(here + (t >> 2) * kPlane) = make_float4(e[t], e[t + 1], e[t + 2], e[t + 3]);
-      beta_next<STD>(be, wt[t], t == 7 ? rb : 1.0f);
+      beta_next<STD>(t, be, wt[t], t == 7 ? rb : 1.0f);
     }
     // input weights flushed to 0: |s| > 126, less the log of b, which is up to 108 - 2 top
     const float smag = max3(max3(fabsf(s[0]), fabsf(s[1]), fabsf(s[2])), max3(fabsf(s[3]), fabsf(s[4]), fabsf(s[5])),
