@@ -12,16 +12,18 @@
 // as logarithms.  A trellis step of the 8 states is 16 multiply-adds and two ex2 for the branch
 // weights, where the (m, s) form of trellis.cuh needs 8 ex2 and about 85 instructions; the
 // extrinsic is one lg2 of each of two 4-term sums.  What limits it is float's exponent range: a
-// probability below 2^-149 becomes 0.  Each step checks that what it computed cannot have lost
-// anything that matters (kLost below); a block that fails goes on in the (m, s) form (siso.cuh),
-// from there or from the start, in a second pass.  LLRs of ordinary channels stay inside the range (extrinsics of
-// about 120 to 170 bits, depending on the parities; eight iterations at 1/3 reach 90 bits at 1 dB, 143 at
-// 2.5 dB); blocks of rate 4/5 that fail their CRC may leave it, scaled-up LLRs do.
+// probability below 2^-149 becomes 0.  Each half-iteration checks, per block, that what was lost cannot
+// matter (kLost below).  A block whose LLRs are about to leave the range of one weight per input (126
+// bits) or whose checks come close goes on in a two-factor form of the same arithmetic, and from there,
+// if it has to, in the (m, s) form (siso.cuh), in passes of their own.  LLRs of ordinary channels stay
+// inside the linear range (extrinsics of about 120 to 170 bits, depending on the parities; eight
+// iterations at 1/3 reach 90 bits at 1 dB, 143 at 2.5 dB); blocks of rate 4/5 that fail their CRC may
+// leave it, scaled-up LLRs do.
 //
-// The linear pass keeps all LLRs in base-2 units (natural LLR * log2(e)).
+// The linear passes keep all LLRs in base-2 units (natural LLR * log2(e)).
 //
-// What bounds it: the issue slots of the SMs, at 2 warps per scheduler (161 instructions per step of a
-// half-iteration, warm-ups included, before most multiplications and multiply-adds went in pairs; the
+// What bounds it: the issue slots of the SMs, at 2 warps per scheduler (about 126 instructions per step of a
+// half-iteration, warm-ups included, 161 before most multiplications and multiply-adds went in pairs; the
 // (m, s) form has about 450).  One warp of 32 windows of 192 steps per CTA, because the shared memory of an
 // SM holds X of 8 of them (7 CTAs with rows of 33 words and a ring of 4 stages were 4 % slower).  4096
 // blocks of K = 6144, 8 iterations: 2.80 ms, 2.89 ms without the pairs, 8.0 ms with the (m, s) kernel that
@@ -95,8 +97,8 @@ __device__ __forceinline__ uint64_t global_ns() {
 //     positions (8 x uint16: 1), systematic (2)
 //   lower SISO: the same of parity 2 and the interleaved positions
 //   alpha checkpoints, one per 8 steps (the extrinsics of the 8 steps replace it): 2 rows8
-//   what the half-iteration read, for a second pass that takes over from there: 2 rows8
-//   (second pass: behind the extrinsics, checkpoints of the (m, s) form, one per 4 steps, and one
+//   what the half-iteration read, for an (m, s) pass that takes over from there: 2 rows8
+//   ((m, s) pass: behind the extrinsics, checkpoints of the (m, s) form, one per 4 steps, and one
 //   more): 4 rows8 + 2
 //   seeds: 2 SISOs x 2 iteration parities x (alpha, beta) x 2 planes: 16
 //   beta at the block end (log values) of the upper and the lower SISO: 4
@@ -113,14 +115,33 @@ __host__ __device__ inline int64_t res_slot_planes(int rows8) { return 16 * stat
 // 2^-|x| of the mass and must be 2^kKept times what was lost anywhere in the block (half an ulp of
 // an x of 64 or more), so that a block passes if
 //   log2(smallest mass) - max |x| >= top + 13 - 150 + kKept.
-// An input weight below 2^-126 is flushed; the paths lost with it weigh 2^-126 times their side of the
-// extrinsic x there, 2^(-126 - x) where x favours the other input.
+// That holds as long as it is metrics that lose, never weights (a lost weight counts relative to metrics
+// of up to 2^top), and as long as nothing grows again that was lost.  So, with q = log2 of the largest parity
+// weight or of its inverse:
+// - While every weight is above 2^-126, |s| + q <= kPlainWeights for the largest |s|, the unlikely input's
+//   weight is one factor (the plain form).  Beyond that, or within kNear of the limit, the block changes to
+//   two factors of 2^(-|s| / 2) applied to the metrics one after the other (WideWeights), good for |s| up
+//   to kWideWeights.  The largest |s| is bounded by the systematic LLR's and the last extrinsic's maxima,
+//   which costs nothing per step.
+// - beta multiplies by the input weights first, the power of two of `weights` among them, and by the
+//   parity weight then, up to 2^q: the plain form leaves q bits less.  (The two-factor form applies the power
+//   of two with the parity; the TS 36.212 code has one product per branch.)
+// - The x of a step leaves out that step's own input weight, and paths that only this weight made
+//   negligible can be all of one side of x.  That takes evidence on the neighbouring steps against this
+//   weight, which shows as a fall of the largest metric: what it falls by within a group beyond kKept bits is
+//   taken off too (falls stay below 20 bits on codewords; blocks that this had to catch had 60 and more).
+// Shown by a restatement on the CPU, 3.2 million blocks of codewords and of noise (AWGN, fading, punctured,
+// saturated and independent LLRs of up to 200 bits, both codes), every half-iteration against 64 bits: those
+// that passed were within 1.1e-5 max(|x + s|, 1 nat).  One factor throughout and neither deduction: off by up
+// to 18 bits.
 constexpr int kKept = 18;
-// A block within kNear of that keeps what its half-iterations read, so that the second pass can go on
-// there (a store more per step: 14 % of the time if all did); one that fails from further off starts again.
+// A block within kNear of either limit of the two-factor form keeps what its half-iterations read, so that the
+// (m, s) pass can go on there (a store more per step); one that fails from further off starts again.
 constexpr float kNear = 40.0f;
 constexpr float kLost = 150.0f - 13.0f - kKept;
-constexpr float kMaxParity = 76.0f;  // larger ones go to the second pass at once
+constexpr float kPlainWeights = 126.0f;
+constexpr float kWideWeights = 250.0f;  // 2^(-|s| / 2) above 2^-126
+constexpr float kMaxParity = 76.0f;  // larger ones (of either sign) go to the (m, s) pass at once
 constexpr int kTopMax = 60;
 // top of a block whose largest parity weight is 2^q: leaves the products of a step 18 bits of growth
 // below 2^126 (on ordinary channels alpha and beta grow by 4 or 5 each)
@@ -145,12 +166,26 @@ __device__ __forceinline__ float max3_nan(float x, float y, float z) {
 // below 2.  (2^(log2(e) Lp) is in the record: a step needs one ex2 here, not two or three, and the
 // unit that computes it was busy for half of the time.)
 struct Weights {
+  static constexpr bool kWide = false;
   float a1, a0, b;
 };
-__device__ __forceinline__ Weights weights(float s, float b) {
-  const float y = __int_as_float(0x7f000000 - (__float_as_int(fmaxf(b, 1.0f)) & 0x7f800000));
+__device__ __forceinline__ float weight_scale(float b) {
+  return __int_as_float(0x7f000000 - (__float_as_int(fmaxf(b, 1.0f)) & 0x7f800000));
+}
+__device__ __forceinline__ void weights(float s, float b, Weights& w) {
+  const float y = weight_scale(b);
   const float x = ex2(-fabsf(s)) * y;
-  return Weights{s < 0.0f ? x : y, s < 0.0f ? y : x, b};
+  w = Weights{s < 0.0f ? x : y, s < 0.0f ? y : x, b};
+}
+// The same in the two-factor form: input 1 / input 0 are c1^2 y / c0^2 y, y the power of two and c of the
+// unlikely input 2^(-|s| / 2).
+struct WideWeights {
+  static constexpr bool kWide = true;
+  float c1, c0, y, b;
+};
+__device__ __forceinline__ void weights(float s, float b, WideWeights& w) {
+  const float h = ex2(-0.5f * fabsf(s));
+  w = WideWeights{s < 0.0f ? h : 1.0f, s < 0.0f ? 1.0f : h, weight_scale(b), b};
 }
 
 // log2(x / y) of positive normal x, y (y < 2^126): the exponents' difference is exact and what is left
@@ -304,7 +339,16 @@ __device__ __forceinline__ void beta_at(int t, const float (&be)[8], const Weigh
   else beta_lin(x, w.b, out);
 }
 
-// One alpha step with weights w, one beta step with weights w scaled by r: step t of a group.
+__device__ __forceinline__ void scale_all(float (&m)[8], float r) {
+  const uint64_t rr = pack2(r, r);
+#pragma unroll
+  for (int s = 0; s < 8; s += 2) unpack2(mul2(pack2(m[s], m[s + 1]), rr), m[s], m[s + 1]);
+}
+// alpha's input weights; one alpha step with weights w, one beta step with weights w of metrics to be scaled
+// by r before the group's first: step t of a group.
+__device__ __forceinline__ void alpha_input(int step, const float (&at)[8], const Weights& w, float (&al)[8]) {
+  alpha_scale_at(step, at, w.a1, w.a0, al);
+}
 template <bool STD>
 __device__ __forceinline__ void alpha_next(int step, float (&al)[8], const Weights& w) {
   float t[8];
@@ -320,10 +364,9 @@ __device__ __forceinline__ void alpha_next(int step, float (&al)[8], const Weigh
   }
 }
 template <bool STD>
-__device__ __forceinline__ void beta_next(int step, float (&be)[8], Weights w, float r) {
-  w.a1 *= r;
-  w.a0 *= r;
+__device__ __forceinline__ void beta_next(int step, float (&be)[8], const Weights& w, float r) {
   float t[8];
+  if (step == 7) scale_all(be, r);
   if constexpr (STD) {
     float g[2][2];
     std_weights(w, g);
@@ -335,6 +378,66 @@ __device__ __forceinline__ void beta_next(int step, float (&be)[8], Weights w, f
 #pragma unroll
     for (int n = 0; n < 8; ++n) be[n] = t[n];
   }
+}
+// The mass of all paths from the sums of alpha beta over the branches with input 1 and 0.
+__device__ __forceinline__ float mass_of(const Weights& w, float s1, float s0) { return fmaf(w.a1, s1, w.a0 * s0); }
+
+// The two-factor form, factor by factor on the metrics, so that no product of weights is formed; beta's
+// power of two goes with the parity (TS 36.212: behind it).
+__device__ __forceinline__ void alpha_input(int, const float (&at)[8], const WideWeights& w, float (&al)[8]) {
+  input_scale(at, w.y, w.y, al);
+  input_scale(al, w.c1, w.c0, al);
+  input_scale(al, w.c1, w.c0, al);
+}
+__device__ __forceinline__ float wide_branch(float m, int input, int par, const WideWeights& w) {
+  if (par) m *= w.b;
+  const float c = input ? w.c1 : w.c0;
+  return m * w.y * c * c;
+}
+template <bool STD>
+__device__ __forceinline__ void alpha_next(int step, float (&al)[8], const WideWeights& w) {
+  float t[8];
+  if constexpr (STD) {
+#pragma unroll
+    for (int n = 0; n < 8; ++n) {
+      const int p0 = 2 * (n & 3);
+      t[n] = wide_branch(al[p0], pred_input<true>(n, 0), pred_parity(n, 0), w) +
+             wide_branch(al[p0 + 1], pred_input<true>(n, 1), pred_parity(n, 1), w);
+    }
+#pragma unroll
+    for (int n = 0; n < 8; ++n) al[n] = t[n];
+  } else {
+    alpha_lin_at(step, al, w.b, t);
+    alpha_input(step, t, w, al);
+  }
+}
+template <bool STD>
+__device__ __forceinline__ void beta_next(int step, float (&be)[8], const WideWeights& w, float r) {
+  float t[8];
+  if (step == 7) scale_all(be, r);
+  if constexpr (STD) {
+#pragma unroll
+    for (int s = 0; s < 8; ++s)
+      t[s] = wide_branch(be[next_state<true>(s, 0)], 0, parity<true>(s, 0), w) +
+             wide_branch(be[next_state<true>(s, 1)], 1, parity<true>(s, 1), w);
+  } else {
+    const float b = w.b * w.y;
+    float x[8];
+    input_scale(be, w.c1, w.c0, x);
+    input_scale(x, w.c1, w.c0, x);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float p = x[j], q = x[j + 4];
+      const float u = fmaf(b, q, w.y * p), v = fmaf(b, p, w.y * q);
+      t[2 * j] = j < 2 ? u : v;
+      t[2 * j + 1] = j < 2 ? v : u;
+    }
+  }
+#pragma unroll
+  for (int n = 0; n < 8; ++n) be[n] = t[n];
+}
+__device__ __forceinline__ float mass_of(const WideWeights& w, float s1, float s0) {
+  return fmaf(w.y * s1 * w.c1, w.c1, w.y * s0 * w.c0 * w.c0);
 }
 
 // log2 metrics (largest 0) <-> scaled probabilities, down to float's smallest (ex2 and lg2 flush
@@ -370,7 +473,7 @@ struct ResCta {
   uint32_t crc_tab[16];  // b(x) x^24 mod g of the 4-bit b
 };
 // Dynamic shared memory of a CTA of NT threads: ResCta; a word per thread, used at the first thread of a
-// block (kWordPar); the ring; X.  Between two passes over the streams the ring is idle, and three words per
+// block (kWordPar); the ring; X.  Between two passes over the streams the ring is idle, and four words per
 // thread in it (kWordExt ..) pass a half-iteration's checks and the CRC between the block's threads.
 extern __shared__ __align__(16) char res_smem[];
 constexpr int kResHead = (sizeof(ResCta) + 15) / 16 * 16;
@@ -403,9 +506,11 @@ template <int NT>
 __device__ __forceinline__ int* res_word(int i) {
   return reinterpret_cast<int*>(res_smem + kResHead + 4 * NT * i);
 }
-constexpr int kWordPar = 0;   // the largest log2 parity weight; infinite: the block is left to the second pass
-constexpr int kWordExt = 1, kWordMass = 2, kWordSyn = 3;  // largest extrinsic, smallest mass, CRC
-constexpr int kSecondPass = 0x7f800000;
+constexpr int kWordPar = 0;   // largest |log2 parity weight|
+// largest extrinsic, smallest mass, CRC, largest fall of alpha
+constexpr int kWordExt = 1, kWordMass = 2, kWordSyn = 3, kWordFall = 4;
+// the passes over a task
+constexpr int kPlain = 0, kWide = 1, kLog = 2;
 template <int NT>
 __device__ __forceinline__ char* res_x() {
   return res_smem + res_x_at(NT);
@@ -450,7 +555,7 @@ struct Slot {
     return (lower ? rows8 : 0) * kRecord + g * kRecord;
   }
   __device__ __forceinline__ uint32_t ckpt(int g) const { return (10 * rows8 + 2 * g) * kPlane; }
-  // (linear pass) what the last half-iteration read, 8 steps
+  // (two-factor form) what the last half-iteration read, 8 steps
   __device__ __forceinline__ uint32_t kept(int g) const { return (12 * rows8 + 2 * g) * kPlane; }
   __device__ __forceinline__ uint32_t seeds(bool lower, int it) const {
     return (16 * rows8 + 2 + (lower ? 8 : 0) + (it & 1 ? 4 : 0)) * kPlane;
@@ -538,10 +643,10 @@ struct Ring {
 
 // One SISO half-iteration of one window in the linear domain, first part: everything that reads
 // other windows' positions of X.  Leaves the alpha checkpoints and the next window's alpha seed,
-// and beta at the window's end in `be`.
-template <bool STD, int NT>
+// and beta at the window's end in `be`; `fall` becomes the largest rescaling of the window's alpha.
+template <bool STD, class W, int NT>
 __device__ __forceinline__ void lin_read(const ResWin& v, const Slot<NT>& m, const int it, const bool lower,
-                                         float (&be)[8]) {
+                                         float (&be)[8], float& fall) {
   constexpr uint32_t kPlane = Slot<NT>::kPlane;
   constexpr uint32_t kRecord = Slot<NT>::kRecord;
   const char* const X = res_x<NT>();
@@ -565,19 +670,20 @@ __device__ __forceinline__ void lin_read(const ResWin& v, const Slot<NT>& m, con
     };
 #pragma unroll
     for (int st = 0; st < kStages; ++st) request(ring.at + st * Ring<NT>::kStage);
+    const float start = __int_as_float((v.top + 127) << 23);
     if (v.lo - G > 0) {
       float sd[8];
       m.ld8(seed_in + 16 * tid, sd);
       lin_from_log(sd, al, v.top);
     } else {
 #pragma unroll
-      for (int n = 0; n < 8; ++n) al[n] = n == 0 ? 1.0f : 0.0f;
+      for (int n = 0; n < 8; ++n) al[n] = n == 0 ? start : 0.0f;
     }
 #pragma unroll 1
     for (; j < gl; ++j) {
       if (j == 0 && v.w == 0) {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) al[k] = k == 0 ? 1.0f : 0.0f;
+        for (int k = 0; k < 8; ++k) al[k] = k == 0 ? start : 0.0f;
       }
       float s[8], b[8];
       ring.read(X, s, b);
@@ -588,11 +694,16 @@ __device__ __forceinline__ void lin_read(const ResWin& v, const Slot<NT>& m, con
         const float o[8] = {al[0], al[4], al[1], al[5], al[2], al[6], al[3], al[7]};  // the pairs of step 0
         m.st8(ck, o);
         ck += 2 * kPlane;
+        fall = fmaxf(fall, r);
       }
       request(ring.at);
       ring.advance();
 #pragma unroll
-      for (int t = 0; t < 8; ++t) alpha_next<STD>(t, al, weights(s[t], b[t]));
+      for (int t = 0; t < 8; ++t) {
+        W w;
+        weights(s[t], b[t], w);
+        alpha_next<STD>(t, al, w);
+      }
     }
   }
   const int tail_at = v.k - (v.lo + v.len);  // steps of the block behind the window
@@ -637,7 +748,11 @@ __device__ __forceinline__ void lin_read(const ResWin& v, const Slot<NT>& m, con
       ring.advance();
       const float r = rescale(be, v.top);
 #pragma unroll
-      for (int t = 7; t >= 0; --t) beta_next<STD>(t, be, weights(s[t], b[t]), t == 7 ? r : 1.0f);
+      for (int t = 7; t >= 0; --t) {
+        W w;
+        weights(s[t], b[t], w);
+        beta_next<STD>(t, be, w, t == 7 ? r : 1.0f);
+      }
     }
     if (tail_at == 0) {
 #pragma unroll
@@ -650,12 +765,12 @@ __device__ __forceinline__ void lin_read(const ResWin& v, const Slot<NT>& m, con
 // extrinsic; the previous window's beta seed is beta at lo + guard.  Replaces the LLRs of the
 // window's own positions in X by the other SISO's input Ls + extrinsic, or (post) by the posterior;
 // with keep_ext the extrinsics stay in the checkpoint planes too, with keep what was read (should a
-// check fail).  Returns the largest |x|
-// and the smallest mass of all paths (0: an overflow or a NaN).
-template <bool STD, int NT>
+// check fail).  Returns the largest |x| and the smallest mass of all paths, less what beta fell by in its
+// group beyond kKept bits (0: an overflow or a NaN).
+template <bool STD, class W, int NT>
 __device__ __forceinline__ float2 lin_write(const ResWin& v, const Slot<NT>& m, const int it, const bool lower,
-                                          float (&be)[8], const float scale, const bool post,
-                                          const bool keep_ext, const bool keep) {
+                                            float (&be)[8], const float scale, const bool post,
+                                            const bool keep_ext, const bool keep) {
   constexpr uint32_t kPlane = Slot<NT>::kPlane;
   constexpr uint32_t kRecord = Slot<NT>::kRecord;
   char* const X = res_x<NT>();
@@ -697,7 +812,7 @@ __device__ __forceinline__ float2 lin_write(const ResWin& v, const Slot<NT>& m, 
     request(ring.at);
     ring.advance();
     char* const here = ck;
-    if (keep) {
+    if (W::kWide && keep) {
       *reinterpret_cast<float4*>(here + kept) = make_float4(s[0], s[1], s[2], s[3]);
       *reinterpret_cast<float4*>(here + kept + kPlane) = make_float4(s[4], s[5], s[6], s[7]);
     }
@@ -709,9 +824,9 @@ __device__ __forceinline__ float2 lin_write(const ResWin& v, const Slot<NT>& m, 
       la = ld(ls);
       lb = ld(ls + kPlane);
     }
-    Weights wt[8];
+    W wt[8];
 #pragma unroll
-    for (int t = 0; t < 8; ++t) wt[t] = weights(s[t], b[t]);
+    for (int t = 0; t < 8; ++t) weights(s[t], b[t], wt[t]);
     const float rb = rescale(be, v.top);
     // A[t]: alpha_{t+1} without its input weight (reference code) or alpha_t (TS 36.212)
     float A[8][8];
@@ -723,7 +838,7 @@ __device__ __forceinline__ float2 lin_write(const ResWin& v, const Slot<NT>& m, 
         if (t < 7) alpha_next<STD>(t, a, wt[t]);
       } else {
         alpha_lin_at(t, a, wt[t].b, A[t]);
-        if (t < 7) alpha_scale_at(t, A[t], wt[t].a1, wt[t].a0, a);
+        if (t < 7) alpha_input(t, A[t], wt[t], a);
       }
     }
     float e[8], xl = 0.0f;
@@ -758,21 +873,13 @@ __device__ __forceinline__ float2 lin_write(const ResWin& v, const Slot<NT>& m, 
       if (t & 1) xl = x;
       else xmax = max3(xmax, fabsf(x), fabsf(xl));
       smax = max3_nan(smax, s1, s0);
-      if (t == 0) mass = min_nan(mass, fmaf(wt[t].a1, s1, wt[t].a0 * s0));
+      // (at t = 7 beta is not rescaled yet)
+      if (t == 7) mass = min_nan(mass, fminf(rb, static_cast<float>(1 << kKept)) * mass_of(wt[t], s1, s0));
       e[t] = scale * x;
       *reinterpret_cast<float*>(X + Ring<NT>::place(places, t)) = base[t] + e[t];
       if (keep_ext && (t & 3) == 0)
         *reinterpret_cast<float4*>(here + (t >> 2) * kPlane) = make_float4(e[t], e[t + 1], e[t + 2], e[t + 3]);
       beta_next<STD>(t, be, wt[t], t == 7 ? rb : 1.0f);
-    }
-    // input weights flushed to 0: |s| > 126, less the log of b, which is up to 108 - 2 top
-    const float smag = max3(max3(fabsf(s[0]), fabsf(s[1]), fabsf(s[2])), max3(fabsf(s[3]), fabsf(s[4]), fabsf(s[5])),
-                            fmaxf(fabsf(s[6]), fabsf(s[7])));
-    if (!(smag <= 2.0f * v.top)) {
-#pragma unroll
-      for (int t = 0; t < 8; ++t)
-        if (fminf(wt[t].a1, wt[t].a0) == 0.0f)
-          mass = min_nan(mass, ex2((s[t] < 0.0f ? -e[t] : e[t]) / scale + static_cast<float>(v.top) + (126.0f - kKept - kLost)));
     }
     if (rec && 8 * j == G) {
       float sd[8];
@@ -784,29 +891,34 @@ __device__ __forceinline__ float2 lin_write(const ResWin& v, const Slot<NT>& m, 
 }
 
 // A half-iteration of the CTA's blocks in the linear domain; `run`: this thread's window takes part.
-// Returns the bits by which its block passed the checks (negative: it did not).
-template <bool STD, int NT>
-__device__ __noinline__ float lin_half(const bool run, const int half, const float scale, const bool post,
-                                       const bool keep_ext, const bool keep) {
+// Returns the bits by which its block passed the checks (negative: it did not) and its largest extrinsic.
+template <bool STD, class W, int NT>
+__device__ __noinline__ float2 lin_half(const bool run, const int half, const float scale, const bool post,
+                                        const bool keep_ext, const bool keep) {
   const ResWin v = res_win<NT>();
   const Slot<NT> m;
   const bool lower = half & 1;
-  float be[8];
-  if (run) lin_read<STD, NT>(v, m, half >> 1, lower, be);
+  float be[8], fall = 1.0f;
+  if (run) lin_read<STD, W, NT>(v, m, half >> 1, lower, be, fall);
   __syncthreads();  // every window has read X (and left its seeds and checkpoints)
   float2 c = make_float2(0.0f, 0.0f);
-  if (run) c = lin_write<STD, NT>(v, m, half >> 1, lower, be, scale, post, keep_ext, keep);
+  if (run) c = lin_write<STD, W, NT>(v, m, half >> 1, lower, be, scale, post, keep_ext, keep);
   __syncthreads();
   res_word<NT>(kWordExt)[threadIdx.x] = 0;
   res_word<NT>(kWordMass)[threadIdx.x] = 0x7f000000;
+  res_word<NT>(kWordFall)[threadIdx.x] = 0x3f800000;
   __syncthreads();
   if (run) {
     atomicMax(res_word<NT>(kWordExt) + v.lane0, __float_as_int(c.x));
     atomicMin(res_word<NT>(kWordMass) + v.lane0, __float_as_int(c.y));
+    atomicMax(res_word<NT>(kWordFall) + v.lane0, __float_as_int(fall));
   }
   __syncthreads();
-  return lg2(__int_as_float(res_word<NT>(kWordMass)[v.lane0])) - __int_as_float(res_word<NT>(kWordExt)[v.lane0]) -
-         (static_cast<float>(v.top) - kLost);
+  const auto word = [&](int i) { return __int_as_float(res_word<NT>(i)[v.lane0]); };
+  const float lost = !STD && !W::kWide ? word(kWordPar) : 0.0f;  // by the plain form's beta
+  return make_float2(lg2(word(kWordMass)) - word(kWordExt) - (static_cast<float>(v.top) - kLost) - lost -
+                         fmaxf(lg2(word(kWordFall)) - static_cast<float>(kKept), 0.0f),
+                     word(kWordExt));
 }
 
 // The extrinsics in the checkpoint planes into X: added to Ls (the other SISO's input), or (post)
@@ -900,9 +1012,10 @@ __device__ __forceinline__ void res_stage_rows(const ResWin& v, const void* src,
 // the upper SISO), the interleaved positions, the tail betas, seeds zero.
 // Each warp stages its windows' rows through shared memory (where X and the ring will be; a row
 // pitch of an odd number of 16-byte words keeps both sides free of bank conflicts).
+// Returns the window's largest systematic |LLR|.
 template <bool STD, int NT>
-__device__ __noinline__ void res_inputs(const ResCb* cb, const float* llr, const uint16_t* perm,
-                                        const bool linear) {
+__device__ __noinline__ float res_inputs(const ResCb* cb, const float* llr, const uint16_t* perm,
+                                         const bool linear) {
   const Slot<NT> m;
   const float unit = linear ? kLog2e : 1.0f;
   const int tid = threadIdx.x;
@@ -947,6 +1060,7 @@ __device__ __noinline__ void res_inputs(const ResCb* cb, const float* llr, const
     __syncwarp();
   }
   const int pitch = 4 * W + 16;
+  float sys = 0.0f;
 #pragma unroll 1
   for (int st = 0; st < 3; ++st) {  // parity 1, parity 2, systematic
     const int which = st == 2 ? 0 : st + 1;
@@ -960,12 +1074,13 @@ __device__ __noinline__ void res_inputs(const ResCb* cb, const float* llr, const
       for (int r = 0; r < v.window; r += 4) {
         float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (r < v.len) x = *reinterpret_cast<const float4*>(row + 4 * r);
-        most = fmaxf(max3(most, x.x, x.y), fmaxf(x.z, x.w));
+        most = max3(max3(most, fabsf(x.x), fabsf(x.y)), fabsf(x.z), fabsf(x.w));
         x = make_float4(unit * x.x, unit * x.y, unit * x.z, unit * x.w);
         if (exp_now) x = make_float4(ex2(x.x), ex2(x.y), ex2(x.z), ex2(x.w));
         m.st(m.record(which == 2, r >> 3) + (which == 0 ? m.kSys : 0) + m.half(r) + 16u * tid, x);
       }
       if (which != 0) atomicMax(res_word<NT>(kWordPar) + v.lane0, __float_as_int(unit * most));
+      else sys = unit * most;
     }
     __syncwarp();
   }
@@ -992,7 +1107,7 @@ __device__ __noinline__ void res_inputs(const ResCb* cb, const float* llr, const
     }
   }
   __syncthreads();
-  if (!mine) return;
+  if (!mine) return 0.0f;
 #pragma unroll 1
   for (int r0 = 0; r0 < v.window; r0 += 32) {
     uint4 q[4];
@@ -1022,6 +1137,7 @@ __device__ __noinline__ void res_inputs(const ResCb* cb, const float* llr, const
       m.st8(m.tail(lower) + 16u * tid, tb);
     }
   }
+  return sys;
 }
 
 // This window's part of its block's CRC24B syndrome of the hard decisions [filler, K)
@@ -1070,7 +1186,7 @@ __device__ __noinline__ void res_outputs(float* dst, const float unit) {
   });
 }
 
-// ---- second pass: blocks whose metrics left float's range, in the (m, s) form of siso.cuh, with
+// ---- (m, s) pass: blocks whose metrics left float's range, in the form of siso.cuh, with
 // X and the planes in natural units ----
 template <bool LOWER, int NT>
 struct SlotAccess {
@@ -1128,11 +1244,17 @@ __device__ __noinline__ void log_half(const float* d0, const int it, const float
   siso_window<kSub, LOWER, STD, false>(cb, io.v.w, io, ck);
 }
 
+// The two-factor form is called through a pointer (volatile: the compiler may not see through it): as a
+// direct call of the kernel it takes registers from the plain form, which needs all of them (12 to 28 bytes
+// of spills in its loops, 4096 blocks of K = 6144 2.82 ms instead of 2.67).
+using LinHalf = float2 (*)(bool, int, float, bool, bool, bool);
+template <bool STD, int NT>
+__device__ volatile LinHalf wide_half = lin_half<STD, WideWeights, NT>;
+
 template <bool STD, int NT>
 __global__ void __launch_bounds__(NT, 256 / NT) resident_kernel(const __grid_constant__ ResArgs p) {
   const int tid = threadIdx.x;
   ResCta& cta = res_cta();
-  int* const left = res_word<NT>(kWordPar);  // kSecondPass: the block (at its first lane) left the linear domain
   for (int task = blockIdx.x; task < p.n_tasks;) {
     if (task == p.stall_task && tid == 0) {  // testing hook: a wait that runs out
       const uint64_t t0 = global_ns();
@@ -1160,7 +1282,7 @@ __global__ void __launch_bounds__(NT, 256 / NT) resident_kernel(const __grid_con
       max_window = max(max_window, o.window);
     }
     const bool mine = cb != nullptr;
-    left[tid] = 0;
+    res_word<NT>(kWordPar)[tid] = 0;
     if (tid == 0) {
       cta.slot = reinterpret_cast<char*>(p.scratch + p.slot * blockIdx.x);
       cta.guard = p.guard;
@@ -1174,26 +1296,36 @@ __global__ void __launch_bounds__(NT, 256 / NT) resident_kernel(const __grid_con
     bool passed = false;
     int used = p.max_iterations;
 
-    // Two passes: all blocks in the linear domain, then the ones that left float's range there, in the
-    // (m, s) form from half-iteration `from`.
-    int from = 0;
+    // Three passes: all blocks in the plain linear form, as far as it goes; what is left in the two-factor
+    // form, from X as it stands; and what that one leaves in the (m, s) form.  `done_in` is the pass that a
+    // block ends in, `from` the half-iteration where that pass takes over.
+    int done_in = kPlain, from = 0;
     float margin = 1000.0f;  // of the block's checks in the last half-iteration
+    float q = 0.0f, sys = 0.0f, most = 0.0f;  // its largest parity and systematic LLR, a bound of |X|
 #pragma unroll 1
-    for (int pass = 0; pass < 2 && p.max_iterations > 0; ++pass) {
-      bool run = mine && (pass == 0 || left[lane0] == kSecondPass);
-      if (pass == 1 && !__syncthreads_or(run)) break;
+    for (int pass = kPlain; pass <= kLog && p.max_iterations > 0; ++pass) {
+      bool run = mine && done_in == pass;
+      if (pass != kPlain && !__syncthreads_or(run)) continue;
       const bool taken = run;
-      res_inputs<STD, NT>(cb, p.llr, p.perm, pass == 0);
-      __syncthreads();
-      if (pass == 1) {
+      if (pass != kWide) {
+        sys = res_inputs<STD, NT>(cb, p.llr, p.perm, pass == kPlain);
+        __syncthreads();
+      }
+      if (pass == kLog) {
         if (run && from > 0) res_restore<NT>(from & 1);
         __syncthreads();
       }
-      if (pass == 0) {
-        const bool wide = run && __int_as_float(left[lane0]) > kMaxParity;
+      if (pass == kPlain) {
+        int* const largest = res_word<NT>(kWordExt);
+        largest[tid] = 0;
         __syncthreads();
-        if (wide) {
-          left[lane0] = kSecondPass;
+        if (run) atomicMax(largest + lane0, __float_as_int(sys));
+        __syncthreads();
+        most = sys = __int_as_float(largest[lane0]);
+        q = __int_as_float(res_word<NT>(kWordPar)[lane0]);
+        __syncthreads();
+        if (run && q > kMaxParity) {
+          done_in = kLog;
           run = false;
         }
       }
@@ -1203,14 +1335,35 @@ __global__ void __launch_bounds__(NT, 256 / NT) resident_kernel(const __grid_con
         const bool lower = half & 1, last_half = half + 1 == 2 * p.max_iterations;
         const bool post_now = lower && (p.early_stop || last_half);
         const float scale = __ldg(p.scale + half);
-        if (pass == 0) {
-          // (a block that fails is left to the second pass)
-          const bool keep = margin < kNear;
-          margin = lin_half<STD, NT>(run, half, scale, post_now, lower && p.early_stop, keep);
-          if (!(margin >= 0.0f) && run) {
-            left[lane0] = kSecondPass;
+        if (pass == kPlain) {
+          if (run && (margin < kNear || !(most + q <= kPlainWeights))) {
+            done_in = kWide;
+            from = half;
             run = false;
-            from = keep ? half : 0;
+          }
+          if (!__syncthreads_or(run)) break;
+          const float2 c = lin_half<STD, Weights, NT>(run, half, scale, post_now, lower && p.early_stop, false);
+          if (run) {
+            margin = c.x;
+            most = sys + fabsf(scale) * c.y;
+            if (!(margin >= 0.0f)) {
+              done_in = kLog;
+              run = false;
+            }
+          }
+        } else if (pass == kWide) {
+          const bool now = run && half >= from;
+          if (!__syncthreads_or(now)) continue;
+          const bool keep = margin < kNear || !(most <= kWideWeights - kNear);
+          const float2 c = wide_half<STD, NT>(now, half, scale, post_now, lower && p.early_stop, keep);
+          if (now) {
+            margin = most > kWideWeights ? -1.0f : c.x;
+            most = sys + fabsf(scale) * c.y;
+            if (!(margin >= 0.0f)) {
+              done_in = kLog;
+              from = keep ? half : 0;
+              run = false;
+            }
           }
         } else {
           if (run && half >= from) {
@@ -1237,9 +1390,9 @@ __global__ void __launch_bounds__(NT, 256 / NT) resident_kernel(const __grid_con
           if (!__syncthreads_or(run)) break;
         }
       }
-      const bool write = taken && (pass == 1 || left[lane0] != kSecondPass);
+      const bool write = taken && done_in == pass;
       res_outputs<NT>(write ? p.post + cb->out + (tid - lane0) * cb->window : nullptr,
-                      pass == 0 ? kLn2 : 1.0f);
+                      pass != kLog ? kLn2 : 1.0f);
       __syncthreads();
     }
     if (mine && tid == lane0) {
