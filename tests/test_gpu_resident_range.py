@@ -104,3 +104,14 @@ def test_no_codeword(tc, decoder, oracle, k, n, size, std):
     ks = [k] * n
     llr = rng.uniform(-size, size, n * 3 * (k + 4)).astype(np.float32)
     _compare(tc, decoder, oracle, ks, llr, 1, std=std)
+
+
+@pytest.mark.parametrize("std", [False, True])
+@pytest.mark.parametrize("iters,guard", [(2, 0), (3, 0), (2, 8)])
+def test_restart_from_the_beginning(tc, decoder, oracle, iters, guard, std):
+    """LLRs three times too large at 1.5 dB: a tenth of the blocks fail their checks all at once at the third
+    half-iteration or later and start again.  Without a guard the first iteration's boundary metrics (all
+    equal) show in the posterior."""
+    ks = [512] * 300
+    llr = std_code_blocks(tc, ks, 1.5, 37)[0] if std else awgn_blocks(tc, ks, 1.5, 37)[0]
+    _compare(tc, decoder, oracle, ks, 3.0 * llr, iters, std=std, guard=guard)

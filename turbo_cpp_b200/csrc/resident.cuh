@@ -1009,13 +1009,14 @@ __device__ __forceinline__ void res_stage_rows(const ResWin& v, const void* src,
 }
 
 // The inputs of a task, in base-2 units with parity weights for the linear pass: the streams' planes, X = the systematic LLRs (the first input of
-// the upper SISO), the interleaved positions, the tail betas, seeds zero.
+// the upper SISO), the interleaved positions, the tail betas; seeds zero if the block starts here (`start`; one
+// that goes on keeps the seeds of the half-iterations before).
 // Each warp stages its windows' rows through shared memory (where X and the ring will be; a row
 // pitch of an odd number of 16-byte words keeps both sides free of bank conflicts).
 // Returns the window's largest systematic |LLR|.
 template <bool STD, int NT>
 __device__ __noinline__ float res_inputs(const ResCb* cb, const float* llr, const uint16_t* perm,
-                                         const bool linear) {
+                                         const bool linear, const bool start) {
   const Slot<NT> m;
   const float unit = linear ? kLog2e : 1.0f;
   const int tid = threadIdx.x;
@@ -1127,7 +1128,7 @@ __device__ __noinline__ float res_inputs(const ResCb* cb, const float* llr, cons
   }
   const uint32_t sd = m.seeds(false, 0) + 16u * tid;
 #pragma unroll 1
-  for (int i = 0; linear && i < 16; ++i) m.st(sd + i * m.kPlane, make_float4(0.0f, 0.0f, 0.0f, 0.0f));
+  for (int i = 0; start && i < 16; ++i) m.st(sd + i * m.kPlane, make_float4(0.0f, 0.0f, 0.0f, 0.0f));
   if (v.k - (v.lo + v.len) <= v.guard) {
 #pragma unroll
     for (int lower = 0; lower < 2; ++lower) {
@@ -1308,7 +1309,7 @@ __global__ void __launch_bounds__(NT, 256 / NT) resident_kernel(const __grid_con
       if (pass != kPlain && !__syncthreads_or(run)) continue;
       const bool taken = run;
       if (pass != kWide) {
-        sys = res_inputs<STD, NT>(cb, p.llr, p.perm, pass == kPlain);
+        sys = res_inputs<STD, NT>(cb, p.llr, p.perm, pass == kPlain, from == 0);
         __syncthreads();
       }
       if (pass == kLog) {
