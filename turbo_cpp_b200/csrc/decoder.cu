@@ -31,21 +31,26 @@ namespace tcb {
 
 namespace {
 
-// The kernel instances: CTAs of 32, 64, 96, 128 or 256 threads.
-constexpr int kResThreads[] = {32, 64, 96, 128, 256};
+// The kernel instances: CTAs of 32, 64, 96, 128 or 256 threads, and of 32 with a compact scratch slot.
+struct ResInstance {
+  int threads;
+  bool compact;
+};
+constexpr ResInstance kResInstances[] = {{32, true}, {32, false}, {64, false}, {96, false}, {128, false}, {256, false}};
 using ResKernel = void (*)(ResArgs);
 template <bool STD>
-ResKernel res_kernel_of(int threads) {
-  switch (threads) {
-    case 32: return resident_kernel<STD, 32>;
-    case 64: return resident_kernel<STD, 64>;
-    case 96: return resident_kernel<STD, 96>;
-    case 128: return resident_kernel<STD, 128>;
-    default: return resident_kernel<STD, 256>;
+ResKernel res_kernel_of(const ResInstance& i) {
+  if (i.compact) return resident_kernel<STD, Shape<32, true>>;
+  switch (i.threads) {
+    case 32: return resident_kernel<STD, Shape<32, false>>;
+    case 64: return resident_kernel<STD, Shape<64, false>>;
+    case 96: return resident_kernel<STD, Shape<96, false>>;
+    case 128: return resident_kernel<STD, Shape<128, false>>;
+    default: return resident_kernel<STD, Shape<256, false>>;
   }
 }
-ResKernel res_kernel(bool std3gpp, int threads) {
-  return std3gpp ? res_kernel_of<true>(threads) : res_kernel_of<false>(threads);
+ResKernel res_kernel(bool std3gpp, const ResInstance& i) {
+  return std3gpp ? res_kernel_of<true>(i) : res_kernel_of<false>(i);
 }
 
 void check(cudaError_t e, const char* what) {
@@ -160,9 +165,9 @@ Decoder::Decoder(int device) : device_(device) {
                         reinterpret_cast<const void*>(siso_plain_kernel<kSub, 2, true>)})
     check(cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 0),
           "carveout attr");
-  for (const int t : kResThreads)
+  for (const ResInstance& i : kResInstances)
     for (const bool std3gpp : {false, true}) {
-      const ResKernel f = res_kernel(std3gpp, t);
+      const ResKernel f = res_kernel(std3gpp, i);
       check(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kResMaxSmem),
             "smem attr");
       check(cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout,
@@ -542,6 +547,8 @@ struct Decoder::Layout {
   std::vector<int32_t> task_first;
   int threads = 0;
   size_t smem = 0;
+  bool compact = false;
+  int64_t slot = 0;  // float4 of a CTA's scratch slot
 };
 
 struct Decoder::Io {
@@ -695,6 +702,7 @@ void Decoder::pack_tasks(const DecodeRequest& rq, Layout& l) const {
   for (size_t i = 0; i < n; ++i) order[start[kQppCount - 1 - qpp_index(l.cbs[i].k)]++] = static_cast<int32_t>(i);
   l.res.resize(n);
   l.task_first.clear();
+  l.slot = 0;
   int lanes = 0, rows = 0;
   size_t x = 0;
   for (size_t j = 0; j < n; ++j) {
@@ -710,9 +718,15 @@ void Decoder::pack_tasks(const DecodeRequest& rq, Layout& l) const {
     l.res[j] = ResCb{d.k, d.filler, d.tab, lanes, d.nwin, d.window, order[j], 0, d.llr, d.out};
     lanes += d.nwin;
     x = std::max(x, res_x_bytes(lanes, rows));
+    l.slot = std::max(l.slot, res_slot(l.threads, rows / 8, lanes));
   }
   l.task_first.push_back(static_cast<int32_t>(n));
   l.smem = x + res_head_bytes(l.threads);
+  // the compact slot where it is less than two thirds of the other (windows from 320 steps on: as fast or
+  // faster there; 600 blocks of K = 6144 at window 512 1.04 ms instead of 1.22, at the full trellis 9.6, 13.4)
+  const int64_t full_slot = res_slot(l.threads, l.max_window / 8, l.threads);
+  l.compact = l.threads == 32 && 3 * l.slot < 2 * full_slot;
+  if (!l.compact) l.slot = full_slot;
   const size_t tasks = l.task_first.size() - 1;
   // windows above 1024 steps leave an SM fewer than 2 warps of lanes (X takes 4 bytes per step):
   // the launch-per-half-iteration kernels run more windows at once, unless the whole batch is one
@@ -725,14 +739,13 @@ void Decoder::run_resident(const DecodeRequest& rq, const Layout& l, const Io& i
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const size_t n = l.res.size();
   const int tasks = static_cast<int>(l.task_first.size()) - 1;
-  const ResKernel f = res_kernel(rq.std3gpp, l.threads);
+  const ResKernel f = res_kernel(rq.std3gpp, {l.threads, l.compact});
   int per_sm = 0;
   check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, l.threads, l.smem), "occupancy");
   const int grid = std::min(tasks, sm_count_ * std::max(per_sm, 1));
 
   ResArgs a{};
-  a.rows8 = l.max_window / 8;
-  a.slot = res_slot_planes(a.rows8) * l.threads;
+  a.slot = l.slot;
   a.scratch = grow<float4>(d_ckpt_, static_cast<size_t>(a.slot) * grid);
   // descriptors: the blocks, the extrinsic scales, the tasks
   const size_t at_scales = n * sizeof(ResCb), n_scales = 2 * static_cast<size_t>(rq.max_iterations);

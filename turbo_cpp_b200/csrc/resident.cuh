@@ -71,7 +71,6 @@ struct ResArgs {
   const uint32_t* xpow;       // x^j mod g_CRC24B, kXpowSize entries, then b(x) x^24 mod g per byte b
   float4* scratch;
   int64_t slot;               // float4 per scratch slot (one slot per CTA of the grid)
-  int rows8;                  // longest window of the call / 8
   int guard;
   int max_iterations;
   int early_stop;
@@ -91,8 +90,8 @@ __device__ __forceinline__ uint64_t global_ns() {
   return t;
 }
 
-// Scratch slot of a CTA of NT threads, in planes of NT float4 (rows8 = longest window / 8, one record
-// per 8 steps):
+// Scratch slot of a CTA, in planes of a float4 per thread or, in the compact layout, per window of the
+// task (rows8 = longest window / 8, one record per 8 steps):
 //   upper SISO: rows8 records of parity 1 (2 planes), the shared-memory byte offsets of the 8
 //     positions (8 x uint16: 1), systematic (2)
 //   lower SISO: the same of parity 2 and the interleaved positions
@@ -102,10 +101,21 @@ __device__ __forceinline__ uint64_t global_ns() {
 //   more): 4 rows8 + 2
 //   seeds: 2 SISOs x 2 iteration parities x (alpha, beta) x 2 planes: 16
 //   beta at the block end (log values) of the upper and the lower SISO: 4
-//   the windows (k, window, nwin, lane0: 4 x uint16): 1
+// and the windows behind them (k, window, nwin, lane0: 4 x uint16, in one float4 per thread).
 // Both SISOs take their places in X from the record, so that they share one copy of the code (with a
 // copy each, the phases that the warps of an SM are in at a time overflow the instruction cache).
-__host__ __device__ inline int64_t res_slot_planes(int rows8) { return 16 * static_cast<int64_t>(rows8) + 23; }
+__host__ __device__ inline int64_t res_slot(int threads, int rows8, int pitch) {  // in float4
+  return (16 * static_cast<int64_t>(rows8) + 22) * pitch + threads;
+}
+// An instance of the kernel.  The compact layout is for one warp with few long windows: X leaves room for
+// 6144 steps of a warp, so a block of full-length windows has one lane of 32 in use, and planes of 32 would
+// take 6.3 MB a CTA, 7.5 GB in all (0.2 MB and 0.23 GB compact).  Its pitch is a run-time value, which the
+// short windows do without: their loops take the planes' offsets as constants.
+template <int THREADS, bool COMPACT>
+struct Shape {
+  static constexpr int kThreads = THREADS;
+  static constexpr bool kCompact = COMPACT;
+};
 
 // Scaling and checks.  The branch weights of a step are below 2, so that the largest metric grows by at
 // most 3 per step; every 8 steps it is set to 2^top, as high as the block's largest parity weight
@@ -466,13 +476,14 @@ __host__ __device__ inline int res_pitch(int lanes) { return lanes % 32 == 0 ? l
 struct ResCta {
   char* slot;          // the CTA's scratch slot
   int guard;
-  int rows8;
+  int rows8;           // longest window of the task / 8
+  uint32_t plane;      // (compact) bytes of a plane of the slot
   uint32_t xs4;        // bytes between the rows of X
   int max_window;      // of the task
   int next_task;
   uint32_t crc_tab[16];  // b(x) x^24 mod g of the 4-bit b
 };
-// Dynamic shared memory of a CTA of NT threads: ResCta; a word per thread, used at the first thread of a
+// Dynamic shared memory of a CTA: ResCta; a word per thread, used at the first thread of a
 // block (kWordPar); the ring; X.  Between two passes over the streams the ring is idle, and four words per
 // thread in it (kWordExt ..) pass a half-iteration's checks and the CRC between the block's threads.
 extern __shared__ __align__(16) char res_smem[];
@@ -496,29 +507,29 @@ struct ResWin {
   int top;                   // of the block
 };
 __device__ __forceinline__ ResCta& res_cta() { return *reinterpret_cast<ResCta*>(res_smem); }
-template <int NT>
+template <class S>
 __device__ __forceinline__ ushort4* res_window() {
   const ResCta& c = *reinterpret_cast<const ResCta*>(res_smem);
-  return reinterpret_cast<ushort4*>(c.slot + (16 * c.rows8 + 22) * 16 * NT);
+  return reinterpret_cast<ushort4*>(c.slot + (16 * c.rows8 + 22) * (S::kCompact ? c.plane : 16u * S::kThreads));
 }
 // word `i` of the per-thread words
-template <int NT>
+template <class S>
 __device__ __forceinline__ int* res_word(int i) {
-  return reinterpret_cast<int*>(res_smem + kResHead + 4 * NT * i);
+  return reinterpret_cast<int*>(res_smem + kResHead + 4 * S::kThreads * i);
 }
 constexpr int kWordPar = 0;   // largest |log2 parity weight|
 // largest extrinsic, smallest mass, CRC, largest fall of alpha
 constexpr int kWordExt = 1, kWordMass = 2, kWordSyn = 3, kWordFall = 4;
 // the passes over a task
 constexpr int kPlain = 0, kWide = 1, kLog = 2;
-template <int NT>
+template <class S>
 __device__ __forceinline__ char* res_x() {
-  return res_smem + res_x_at(NT);
+  return res_smem + res_x_at(S::kThreads);
 }
-template <int NT>
+template <class S>
 __device__ __forceinline__ ResWin res_win() {
   const ResCta& c = res_cta();
-  const ushort4 t = res_window<NT>()[threadIdx.x];
+  const ushort4 t = res_window<S>()[threadIdx.x];
   ResWin v;
   v.tid = threadIdx.x;
   v.k = t.x;
@@ -532,7 +543,7 @@ __device__ __forceinline__ ResWin res_win() {
   v.prev = v.w > 0 ? v.tid - 1 : v.tid;
   v.next = v.w + 1 < v.nwin ? v.tid + 1 : v.tid;
   v.xs4 = c.xs4;
-  v.top = res_top(__int_as_float(res_word<NT>(kWordPar)[v.lane0]));
+  v.top = res_top(__int_as_float(res_word<S>(kWordPar)[v.lane0]));
   return v;
 }
 
@@ -542,47 +553,55 @@ __device__ __forceinline__ float lds(const char* x, uint32_t off) {
 
 // The scratch slot of the CTA, addressed by 32-bit byte offsets.  Plain loads and stores: what other
 // lanes wrote is read after a barrier, never through the read-only path.
-template <int NT>
-struct Slot {
-  static constexpr uint32_t kPlane = 16u * NT;
+template <class S, bool = S::kCompact>
+struct PlanePitch {
+  static constexpr uint32_t plane = 16u * S::kThreads;
+};
+template <class S>
+struct PlanePitch<S, true> {
+  uint32_t plane;
+  __device__ __forceinline__ PlanePitch() : plane(res_cta().plane) {}
+};
+template <class S>
+struct Slot : PlanePitch<S> {
+  using PlanePitch<S>::plane;
   char* base;
   uint32_t rows8;
   __device__ __forceinline__ Slot() : base(res_cta().slot), rows8(res_cta().rows8) {}
   // byte offset of an 8-step record of the upper / lower SISO, of the checkpoint of such a group, of
   // the seeds of a SISO written in iterations of a parity, of a SISO's tail
-  static constexpr uint32_t kRecord = 5 * kPlane;
   __device__ __forceinline__ uint32_t record(bool lower, int g) const {
-    return (lower ? rows8 : 0) * kRecord + g * kRecord;
+    return (lower ? rows8 : 0) * (5 * plane) + g * (5 * plane);
   }
-  __device__ __forceinline__ uint32_t ckpt(int g) const { return (10 * rows8 + 2 * g) * kPlane; }
+  __device__ __forceinline__ uint32_t ckpt(int g) const { return (10 * rows8 + 2 * g) * plane; }
   // (two-factor form) what the last half-iteration read, 8 steps
-  __device__ __forceinline__ uint32_t kept(int g) const { return (12 * rows8 + 2 * g) * kPlane; }
+  __device__ __forceinline__ uint32_t kept(int g) const { return (12 * rows8 + 2 * g) * plane; }
   __device__ __forceinline__ uint32_t seeds(bool lower, int it) const {
-    return (16 * rows8 + 2 + (lower ? 8 : 0) + (it & 1 ? 4 : 0)) * kPlane;
+    return (16 * rows8 + 2 + (lower ? 8 : 0) + (it & 1 ? 4 : 0)) * plane;
   }
   __device__ __forceinline__ uint32_t tail(bool lower) const {
-    return (16 * rows8 + 18 + (lower ? 2 : 0)) * kPlane;
+    return (16 * rows8 + 18 + (lower ? 2 : 0)) * plane;
   }
   // planes of a record
-  static constexpr uint32_t kIndex = 2 * kPlane;
-  static constexpr uint32_t kSys = 3 * kPlane;
+  __device__ __forceinline__ uint32_t index() const { return 2 * plane; }
+  __device__ __forceinline__ uint32_t sys() const { return 3 * plane; }
   __device__ __forceinline__ float4 ld(uint32_t o) const { return *reinterpret_cast<const float4*>(base + o); }
   __device__ __forceinline__ uint2 ld2(uint32_t o) const { return *reinterpret_cast<const uint2*>(base + o); }
   __device__ __forceinline__ void st(uint32_t o, float4 v) const { *reinterpret_cast<float4*>(base + o) = v; }
   __device__ __forceinline__ void st2(uint32_t o, uint2 v) const { *reinterpret_cast<uint2*>(base + o) = v; }
   __device__ __forceinline__ void ld8(uint32_t o, float (&v)[8]) const {
-    const float4 x = ld(o), y = ld(o + kPlane);
+    const float4 x = ld(o), y = ld(o + plane);
     v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
   }
   __device__ __forceinline__ void st8(uint32_t o, const float (&v)[8]) const {
     st(o, make_float4(v[0], v[1], v[2], v[3]));
-    st(o + kPlane, make_float4(v[4], v[5], v[6], v[7]));
+    st(o + plane, make_float4(v[4], v[5], v[6], v[7]));
   }
   // offset of 4 steps' entry within a stream of 2 planes per record
-  static __device__ __forceinline__ uint32_t half(int r) { return (r >> 2 & 1) * kPlane; }
+  __device__ __forceinline__ uint32_t half(int r) const { return (r >> 2 & 1) * plane; }
   // shared-memory offsets of the 4 positions from row r of a column
   __device__ __forceinline__ uint2 positions(bool lower, int r, int col) const {
-    return ld2(record(lower, r >> 3) + kIndex + 16 * col + ((r & 4) << 1));
+    return ld2(record(lower, r >> 3) + index() + 16 * col + ((r & 4) << 1));
   }
 };
 
@@ -591,8 +610,9 @@ __device__ __forceinline__ void put(float (&b)[8], float4 x, float4 y) {
 }
 
 // The ring: requests go round the stages in order, and so do the reads.
-template <int NT>
+template <class S>
 struct Ring {
+  static constexpr uint32_t NT = S::kThreads;
   static constexpr uint32_t kStage = 16u * NT * kEntries;
   uint32_t smem, first, at;  // shared-memory address of res_smem; the thread's entry in stage 0 and in
                              // the next stage, bytes from there
@@ -602,12 +622,12 @@ struct Ring {
     at = first;
   }
   // requests the parity planes and the positions of the record at `src` into the stage at `to`
-  __device__ __forceinline__ void request(uint32_t to, const char* src, bool any) const {
+  __device__ __forceinline__ void request(uint32_t to, const char* src, const uint32_t plane, bool any) const {
     if (any) {
       to += smem;
       copy(to, src);
-      copy(to + 16u * NT, src + 16 * NT);
-      copy(to + 32u * NT, src + 32 * NT);
+      copy(to + 16u * NT, src + plane);
+      copy(to + 32u * NT, src + 2 * plane);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
@@ -644,12 +664,11 @@ struct Ring {
 // One SISO half-iteration of one window in the linear domain, first part: everything that reads
 // other windows' positions of X.  Leaves the alpha checkpoints and the next window's alpha seed,
 // and beta at the window's end in `be`; `fall` becomes the largest rescaling of the window's alpha.
-template <bool STD, class W, int NT>
-__device__ __forceinline__ void lin_read(const ResWin& v, const Slot<NT>& m, const int it, const bool lower,
+template <bool STD, class W, class S>
+__device__ __forceinline__ void lin_read(const ResWin& v, const Slot<S>& m, const int it, const bool lower,
                                          float (&be)[8], float& fall) {
-  constexpr uint32_t kPlane = Slot<NT>::kPlane;
-  constexpr uint32_t kRecord = Slot<NT>::kRecord;
-  const char* const X = res_x<NT>();
+  const uint32_t kPlane = m.plane, kRecord = 5 * m.plane;
+  const char* const X = res_x<S>();
   const int tid = v.tid, G = v.guard;
   const uint32_t seed_in = m.seeds(lower, it), seed_out = m.seeds(lower, it + 1);
   float al[8];
@@ -660,16 +679,16 @@ __device__ __forceinline__ void lin_read(const ResWin& v, const Slot<NT>& m, con
     const int row0 = j < 0 ? v.window - G : 0, col0 = j < 0 ? v.prev : tid;
     uint32_t ck = m.ckpt(0) + 16u * tid;
     // i, src: the group that is requested next (the window's own first one follows the warm-up's last)
-    Ring<NT> ring;
+    Ring<S> ring;
     int i = j;
     const char* const own = m.base + m.record(lower, 0) + 16u * tid;
     const char* src = m.base + m.record(lower, row0 >> 3) + 16u * col0;
     auto request = [&](uint32_t to) {
-      ring.request(to, src, i < gl);
+      ring.request(to, src, kPlane, i < gl);
       src = ++i == 0 ? own : src + kRecord;
     };
 #pragma unroll
-    for (int st = 0; st < kStages; ++st) request(ring.at + st * Ring<NT>::kStage);
+    for (int st = 0; st < kStages; ++st) request(ring.at + st * Ring<S>::kStage);
     const float start = __int_as_float((v.top + 127) << 23);
     if (v.lo - G > 0) {
       float sd[8];
@@ -726,16 +745,16 @@ __device__ __forceinline__ void lin_read(const ResWin& v, const Slot<NT>& m, con
 #pragma unroll
   for (int n = 0; n < 8; ++n) be[n] = tb[n];
   if (v.nwin > 1 && G > 0) {
-    Ring<NT> ring;
+    Ring<S> ring;
     int j = (G >> 3) - 1, i = j;
     const char* src = m.base + m.record(lower, j) + 16u * v.next;
     auto request = [&](uint32_t to) {
-      ring.request(to, src, i >= 0);
+      ring.request(to, src, kPlane, i >= 0);
       --i;
       src -= kRecord;
     };
 #pragma unroll
-    for (int st = 0; st < kStages; ++st) request(ring.at + st * Ring<NT>::kStage);
+    for (int st = 0; st < kStages; ++st) request(ring.at + st * Ring<S>::kStage);
 #pragma unroll 1
     for (; j >= 0; --j) {
       if (8 * (j + 1) == tail_at) {
@@ -767,30 +786,29 @@ __device__ __forceinline__ void lin_read(const ResWin& v, const Slot<NT>& m, con
 // with keep_ext the extrinsics stay in the checkpoint planes too, with keep what was read (should a
 // check fail).  Returns the largest |x| and the smallest mass of all paths, less what beta fell by in its
 // group beyond kKept bits (0: an overflow or a NaN).
-template <bool STD, class W, int NT>
-__device__ __forceinline__ float2 lin_write(const ResWin& v, const Slot<NT>& m, const int it, const bool lower,
+template <bool STD, class W, class S>
+__device__ __forceinline__ float2 lin_write(const ResWin& v, const Slot<S>& m, const int it, const bool lower,
                                             float (&be)[8], const float scale, const bool post,
                                             const bool keep_ext, const bool keep) {
-  constexpr uint32_t kPlane = Slot<NT>::kPlane;
-  constexpr uint32_t kRecord = Slot<NT>::kRecord;
-  char* const X = res_x<NT>();
+  const uint32_t kPlane = m.plane, kRecord = 5 * m.plane;
+  char* const X = res_x<S>();
   const int tid = v.tid, G = v.guard;
   const uint32_t seed_out = m.seeds(lower, it + 1) + 2 * kPlane + 16 * v.prev;
   float xmax = 0.0f, smax = 0.0f, mass = 3.0e38f;  // checks
   const bool rec = v.w > 0 && G <= v.len;
-  Ring<NT> ring;
+  Ring<S> ring;
   int j = (v.len >> 3) - 1, i = j;
   const char* src = m.base + m.record(lower, j) + 16u * tid;
-  const char* ls = src + Slot<NT>::kSys;
+  const char* ls = src + m.sys();
   char* ck = m.base + m.ckpt(j) + 16u * tid;
   const uint32_t kept = m.kept(0) - m.ckpt(0);
   auto request = [&](uint32_t to) {
-    ring.request(to, src, i >= 0);
+    ring.request(to, src, kPlane, i >= 0);
     --i;
     src -= kRecord;
   };
 #pragma unroll
-  for (int st = 0; st < kStages; ++st) request(ring.at + st * Ring<NT>::kStage);
+  for (int st = 0; st < kStages; ++st) request(ring.at + st * Ring<S>::kStage);
   auto ld = [](const char* p) { return *reinterpret_cast<const float4*>(p); };
   float4 ca = ld(ck), cb = ld(ck + kPlane), la = ld(ls), lb = ld(ls + kPlane);
   if (rec && v.len == G) {
@@ -876,7 +894,7 @@ __device__ __forceinline__ float2 lin_write(const ResWin& v, const Slot<NT>& m, 
       // (at t = 7 beta is not rescaled yet)
       if (t == 7) mass = min_nan(mass, fminf(rb, static_cast<float>(1 << kKept)) * mass_of(wt[t], s1, s0));
       e[t] = scale * x;
-      *reinterpret_cast<float*>(X + Ring<NT>::place(places, t)) = base[t] + e[t];
+      *reinterpret_cast<float*>(X + Ring<S>::place(places, t)) = base[t] + e[t];
       if (keep_ext && (t & 3) == 0)
         *reinterpret_cast<float4*>(here + (t >> 2) * kPlane) = make_float4(e[t], e[t + 1], e[t + 2], e[t + 3]);
       beta_next<STD>(t, be, wt[t], t == 7 ? rb : 1.0f);
@@ -892,29 +910,29 @@ __device__ __forceinline__ float2 lin_write(const ResWin& v, const Slot<NT>& m, 
 
 // A half-iteration of the CTA's blocks in the linear domain; `run`: this thread's window takes part.
 // Returns the bits by which its block passed the checks (negative: it did not) and its largest extrinsic.
-template <bool STD, class W, int NT>
+template <bool STD, class W, class S>
 __device__ __noinline__ float2 lin_half(const bool run, const int half, const float scale, const bool post,
                                         const bool keep_ext, const bool keep) {
-  const ResWin v = res_win<NT>();
-  const Slot<NT> m;
+  const ResWin v = res_win<S>();
+  const Slot<S> m;
   const bool lower = half & 1;
   float be[8], fall = 1.0f;
-  if (run) lin_read<STD, W, NT>(v, m, half >> 1, lower, be, fall);
+  if (run) lin_read<STD, W, S>(v, m, half >> 1, lower, be, fall);
   __syncthreads();  // every window has read X (and left its seeds and checkpoints)
   float2 c = make_float2(0.0f, 0.0f);
-  if (run) c = lin_write<STD, W, NT>(v, m, half >> 1, lower, be, scale, post, keep_ext, keep);
+  if (run) c = lin_write<STD, W, S>(v, m, half >> 1, lower, be, scale, post, keep_ext, keep);
   __syncthreads();
-  res_word<NT>(kWordExt)[threadIdx.x] = 0;
-  res_word<NT>(kWordMass)[threadIdx.x] = 0x7f000000;
-  res_word<NT>(kWordFall)[threadIdx.x] = 0x3f800000;
+  res_word<S>(kWordExt)[threadIdx.x] = 0;
+  res_word<S>(kWordMass)[threadIdx.x] = 0x7f000000;
+  res_word<S>(kWordFall)[threadIdx.x] = 0x3f800000;
   __syncthreads();
   if (run) {
-    atomicMax(res_word<NT>(kWordExt) + v.lane0, __float_as_int(c.x));
-    atomicMin(res_word<NT>(kWordMass) + v.lane0, __float_as_int(c.y));
-    atomicMax(res_word<NT>(kWordFall) + v.lane0, __float_as_int(fall));
+    atomicMax(res_word<S>(kWordExt) + v.lane0, __float_as_int(c.x));
+    atomicMin(res_word<S>(kWordMass) + v.lane0, __float_as_int(c.y));
+    atomicMax(res_word<S>(kWordFall) + v.lane0, __float_as_int(fall));
   }
   __syncthreads();
-  const auto word = [&](int i) { return __int_as_float(res_word<NT>(i)[v.lane0]); };
+  const auto word = [&](int i) { return __int_as_float(res_word<S>(i)[v.lane0]); };
   const float lost = !STD && !W::kWide ? word(kWordPar) : 0.0f;  // by the plain form's beta
   return make_float2(lg2(word(kWordMass)) - word(kWordExt) - (static_cast<float>(v.top) - kLost) - lost -
                          fmaxf(lg2(word(kWordFall)) - static_cast<float>(kKept), 0.0f),
@@ -923,11 +941,11 @@ __device__ __noinline__ float2 lin_half(const bool run, const int half, const fl
 
 // The extrinsics in the checkpoint planes into X: added to Ls (the other SISO's input), or (post)
 // to what stands there (the posterior).
-template <int NT>
+template <class S>
 __device__ __noinline__ void put_extrinsics(const bool lower, const bool post) {
-  const ResWin v = res_win<NT>();
-  const Slot<NT> m;
-  char* const X = res_x<NT>();
+  const ResWin v = res_win<S>();
+  const Slot<S> m;
+  char* const X = res_x<S>();
   // 32 steps at a time, all loads before any use (rows behind the window repeat its last ones)
   constexpr int kPart = 4;
 #pragma unroll 1
@@ -938,15 +956,15 @@ __device__ __noinline__ void put_extrinsics(const bool lower, const bool post) {
     for (int i = 0; i < kPart; ++i) {
       const int g = min(r0 + 8 * i, v.len - 8) >> 3;
       m.ld8(m.ckpt(g) + 16 * v.tid, e[i]);
-      m.ld8(m.record(lower, g) + m.kSys + 16 * v.tid, l[i]);
-      q[i] = *reinterpret_cast<const uint4*>(m.base + m.record(lower, g) + m.kIndex + 16 * v.tid);
+      m.ld8(m.record(lower, g) + m.sys() + 16 * v.tid, l[i]);
+      q[i] = *reinterpret_cast<const uint4*>(m.base + m.record(lower, g) + m.index() + 16 * v.tid);
     }
 #pragma unroll
     for (int i = 0; i < kPart; ++i) {
       if (r0 + 8 * i >= v.len) break;
 #pragma unroll
       for (int t = 0; t < 8; ++t) {
-        float* d = reinterpret_cast<float*>(X + Ring<NT>::place(q[i], t));
+        float* d = reinterpret_cast<float*>(X + Ring<S>::place(q[i], t));
         *d = (post ? *d : l[i][t]) + e[i][t];
       }
     }
@@ -954,18 +972,18 @@ __device__ __noinline__ void put_extrinsics(const bool lower, const bool post) {
 }
 
 // X of this thread's window as the half-iteration that failed had it, in natural units.
-template <int NT>
+template <class S>
 __device__ __noinline__ void res_restore(const bool lower) {
-  const ResWin v = res_win<NT>();
-  const Slot<NT> m;
-  char* const X = res_x<NT>();
+  const ResWin v = res_win<S>();
+  const Slot<S> m;
+  char* const X = res_x<S>();
 #pragma unroll 2
   for (int g = 0; g < v.len >> 3; ++g) {
     float s[8];
     m.ld8(m.kept(g) + 16 * v.tid, s);
-    const uint4 q = *reinterpret_cast<const uint4*>(m.base + m.record(lower, g) + m.kIndex + 16 * v.tid);
+    const uint4 q = *reinterpret_cast<const uint4*>(m.base + m.record(lower, g) + m.index() + 16 * v.tid);
 #pragma unroll
-    for (int t = 0; t < 8; ++t) *reinterpret_cast<float*>(X + Ring<NT>::place(q, t)) = kLn2 * s[t];
+    for (int t = 0; t < 8; ++t) *reinterpret_cast<float*>(X + Ring<S>::place(q, t)) = kLn2 * s[t];
   }
 }
 
@@ -1014,16 +1032,16 @@ __device__ __forceinline__ void res_stage_rows(const ResWin& v, const void* src,
 // Each warp stages its windows' rows through shared memory (where X and the ring will be; a row
 // pitch of an odd number of 16-byte words keeps both sides free of bank conflicts).
 // Returns the window's largest systematic |LLR|.
-template <bool STD, int NT>
+template <bool STD, class S>
 __device__ __noinline__ float res_inputs(const ResCb* cb, const float* llr, const uint16_t* perm,
                                          const bool linear, const bool start) {
-  const Slot<NT> m;
+  const Slot<S> m;
   const float unit = linear ? kLog2e : 1.0f;
   const int tid = threadIdx.x;
   const bool mine = cb != nullptr;
-  const ResWin v = res_win<NT>();
-  char* const X = res_x<NT>();
-  char* const stage = res_smem + res_ring_at(NT);
+  const ResWin v = res_win<S>();
+  char* const X = res_x<S>();
+  char* const stage = res_smem + res_ring_at(S::kThreads);
   const int W = res_cta().max_window;
   const float* const d0 = mine ? llr + cb->llr : nullptr;
   __syncthreads();
@@ -1050,10 +1068,10 @@ __device__ __noinline__ float res_inputs(const ResCb* cb, const float* llr, cons
 #pragma unroll
           for (int t = 0; t < 8; ++t) o[t] = 4u * tid;
         }
-        *reinterpret_cast<uint4*>(m.base + m.record(true, r >> 3) + m.kIndex + 16u * tid) =
+        *reinterpret_cast<uint4*>(m.base + m.record(true, r >> 3) + m.index() + 16u * tid) =
             make_uint4(o[0] | o[1] << 16, o[2] | o[3] << 16, o[4] | o[5] << 16, o[6] | o[7] << 16);
         const uint32_t own = r * v.xs4 + 4u * tid, two = own | own << 16, step = v.xs4 | v.xs4 << 16;
-        *reinterpret_cast<uint4*>(m.base + m.record(false, r >> 3) + m.kIndex + 16u * tid) =
+        *reinterpret_cast<uint4*>(m.base + m.record(false, r >> 3) + m.index() + 16u * tid) =
             make_uint4(two + (v.xs4 << 16), two + 2 * step + (v.xs4 << 16), two + 4 * step + (v.xs4 << 16),
                        two + 6 * step + (v.xs4 << 16));
       }
@@ -1065,7 +1083,7 @@ __device__ __noinline__ float res_inputs(const ResCb* cb, const float* llr, cons
 #pragma unroll 1
   for (int st = 0; st < 3; ++st) {  // parity 1, parity 2, systematic
     const int which = st == 2 ? 0 : st + 1;
-    if (NT > 32) __syncthreads();  // (pitches differ: a row may lie in another warp's part)
+    if (S::kThreads > 32) __syncthreads();  // (pitches differ: a row may lie in another warp's part)
     res_stage_rows<4>(v, mine ? d0 + which * (v.k + 4) + v.lo : nullptr, stage, pitch);
     if (mine) {
       const char* row = stage + tid * pitch;
@@ -1078,9 +1096,9 @@ __device__ __noinline__ float res_inputs(const ResCb* cb, const float* llr, cons
         most = max3(max3(most, fabsf(x.x), fabsf(x.y)), fabsf(x.z), fabsf(x.w));
         x = make_float4(unit * x.x, unit * x.y, unit * x.z, unit * x.w);
         if (exp_now) x = make_float4(ex2(x.x), ex2(x.y), ex2(x.z), ex2(x.w));
-        m.st(m.record(which == 2, r >> 3) + (which == 0 ? m.kSys : 0) + m.half(r) + 16u * tid, x);
+        m.st(m.record(which == 2, r >> 3) + (which == 0 ? m.sys() : 0) + m.half(r) + 16u * tid, x);
       }
-      if (which != 0) atomicMax(res_word<NT>(kWordPar) + v.lane0, __float_as_int(unit * most));
+      if (which != 0) atomicMax(res_word<S>(kWordPar) + v.lane0, __float_as_int(unit * most));
       else sys = unit * most;
     }
     __syncwarp();
@@ -1094,7 +1112,7 @@ __device__ __noinline__ float res_inputs(const ResCb* cb, const float* llr, cons
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const int r = min(r0 + 4 * i, v.len - 4);
-        x[i] = m.ld(m.record(false, r >> 3) + m.kSys + m.half(r) + 16 * tid);
+        x[i] = m.ld(m.record(false, r >> 3) + m.sys() + m.half(r) + 16 * tid);
       }
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
@@ -1115,20 +1133,20 @@ __device__ __noinline__ float res_inputs(const ResCb* cb, const float* llr, cons
 #pragma unroll
     for (int i = 0; i < 4; ++i)
       q[i] = *reinterpret_cast<const uint4*>(
-          m.base + m.record(true, min(r0 + 8 * i, v.window - 8) >> 3) + m.kIndex + 16u * tid);
+          m.base + m.record(true, min(r0 + 8 * i, v.window - 8) >> 3) + m.index() + 16u * tid);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       if (r0 + 8 * i >= v.window) break;
-      const uint32_t at = m.record(true, (r0 >> 3) + i) + m.kSys + 16u * tid;
+      const uint32_t at = m.record(true, (r0 >> 3) + i) + m.sys() + 16u * tid;
       m.st(at, make_float4(lds(X, q[i].x & 0xffffu), lds(X, q[i].x >> 16), lds(X, q[i].y & 0xffffu),
                            lds(X, q[i].y >> 16)));
-      m.st(at + m.kPlane, make_float4(lds(X, q[i].z & 0xffffu), lds(X, q[i].z >> 16),
+      m.st(at + m.plane, make_float4(lds(X, q[i].z & 0xffffu), lds(X, q[i].z >> 16),
                                       lds(X, q[i].w & 0xffffu), lds(X, q[i].w >> 16)));
     }
   }
   const uint32_t sd = m.seeds(false, 0) + 16u * tid;
 #pragma unroll 1
-  for (int i = 0; start && i < 16; ++i) m.st(sd + i * m.kPlane, make_float4(0.0f, 0.0f, 0.0f, 0.0f));
+  for (int i = 0; start && i < 16; ++i) m.st(sd + i * m.plane, make_float4(0.0f, 0.0f, 0.0f, 0.0f));
   if (v.k - (v.lo + v.len) <= v.guard) {
 #pragma unroll
     for (int lower = 0; lower < 2; ++lower) {
@@ -1143,10 +1161,10 @@ __device__ __noinline__ float res_inputs(const ResCb* cb, const float* llr, cons
 
 // This window's part of its block's CRC24B syndrome of the hard decisions [filler, K)
 // (lte_turbo.cpp:792-804): the window's bits modulo g 4 at a time, times x^(steps behind it).
-template <int NT>
+template <class S>
 __device__ __noinline__ void res_crc(const uint32_t* xpow, const int filler) {
-  const ResWin v = res_win<NT>();
-  const char* const X = res_x<NT>();
+  const ResWin v = res_win<S>();
+  const char* const X = res_x<S>();
   const uint32_t* const tab = res_cta().crc_tab;
   uint32_t c = 0, off = 4u * v.tid;
 #pragma unroll 4
@@ -1164,16 +1182,16 @@ __device__ __noinline__ void res_crc(const uint32_t* xpow, const int filler) {
   const uint32_t* xp = xpow + (v.k - (v.lo + v.len));
 #pragma unroll
   for (int b = 0; b < 24; ++b) z ^= (c >> b) & 1u ? __ldg(xp + b) : 0u;
-  atomicXor(reinterpret_cast<uint32_t*>(res_word<NT>(kWordSyn)) + v.lane0, z);
+  atomicXor(reinterpret_cast<uint32_t*>(res_word<S>(kWordSyn)) + v.lane0, z);
 }
 
 // The posteriors in X, times `unit`, of the windows whose lane has a `dst` to there, each warp its own
 // windows.
-template <int NT>
+template <class S>
 __device__ __noinline__ void res_outputs(float* dst, const float unit) {
-  const ResWin v = res_win<NT>();
+  const ResWin v = res_win<S>();
   const int lane = threadIdx.x & 31;
-  const char* const X = res_x<NT>() + 4 * (v.tid - lane);
+  const char* const X = res_x<S>() + 4 * (v.tid - lane);
   res_for_blocks(v, [&](int l, int steps, int window) {
     float* const p = reinterpret_cast<float*>(
         __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(dst), l));
@@ -1189,10 +1207,10 @@ __device__ __noinline__ void res_outputs(float* dst, const float unit) {
 
 // ---- (m, s) pass: blocks whose metrics left float's range, in the form of siso.cuh, with
 // X and the planes in natural units ----
-template <bool LOWER, int NT>
+template <bool LOWER, class S>
 struct SlotAccess {
   ResWin v;
-  Slot<NT> m;
+  Slot<S> m;
   uint32_t seed_in, seed_out;
   float factor;
   const float* d0;
@@ -1208,7 +1226,7 @@ struct SlotAccess {
       row -= v.window;
       ++col;
     }
-    const char* const X = res_x<NT>();
+    const char* const X = res_x<S>();
     const uint2 w = m.positions(LOWER, row, col);
     return Raw4{make_float4(lds(X, w.x & 0xffffu), lds(X, w.x >> 16), lds(X, w.y & 0xffffu), lds(X, w.y >> 16)),
                 make_float4(0.0f, 0.0f, 0.0f, 0.0f),
@@ -1216,10 +1234,10 @@ struct SlotAccess {
   }
   __device__ __forceinline__ Raw8 raw8(int q) const { return Raw8{raw4(q), raw4(q + 4)}; }
   __device__ __forceinline__ void load_seed(bool beta, float (&x)[8]) const {
-    m.ld8(seed_in + (beta ? 2 * m.kPlane : 0) + 16 * v.tid, x);
+    m.ld8(seed_in + (beta ? 2 * m.plane : 0) + 16 * v.tid, x);
   }
   __device__ __forceinline__ void store_seed(bool beta, const float (&x)[8]) const {
-    m.st8(seed_out + (beta ? 2 * m.kPlane + 16 * v.prev : 16 * v.next), x);
+    m.st8(seed_out + (beta ? 2 * m.plane + 16 * v.prev : 16 * v.next), x);
   }
   __device__ __forceinline__ uint2 targets(int) const { return make_uint2(0, 0); }
   __device__ __forceinline__ void put(int q, int, float e, float) const {
@@ -1229,10 +1247,10 @@ struct SlotAccess {
 };
 
 // A half-iteration of this thread's window: reads X, leaves the extrinsics in the checkpoint planes.
-template <bool LOWER, bool STD, int NT>
+template <bool LOWER, bool STD, class S>
 __device__ __noinline__ void log_half(const float* d0, const int it, const float scale) {
-  SlotAccess<LOWER, NT> io;
-  io.v = res_win<NT>();
+  SlotAccess<LOWER, S> io;
+  io.v = res_win<S>();
   io.seed_in = io.m.seeds(LOWER, it);
   io.seed_out = io.m.seeds(LOWER, it + 1);
   io.factor = scale;
@@ -1241,7 +1259,8 @@ __device__ __noinline__ void log_half(const float* d0, const int it, const float
   cb.k = io.v.k;
   cb.nwin = io.v.nwin;
   cb.window = io.v.window;
-  const CkptStrided ck{reinterpret_cast<float4*>(io.m.base) + 12 * io.m.rows8 * NT, NT, io.v.tid};
+  const int pitch = io.m.plane / 16;
+  const CkptStrided ck{reinterpret_cast<float4*>(io.m.base) + 12 * io.m.rows8 * pitch, pitch, io.v.tid};
   siso_window<kSub, LOWER, STD, false>(cb, io.v.w, io, ck);
 }
 
@@ -1249,11 +1268,11 @@ __device__ __noinline__ void log_half(const float* d0, const int it, const float
 // direct call of the kernel it takes registers from the plain form, which needs all of them (12 to 28 bytes
 // of spills in its loops, 4096 blocks of K = 6144 2.82 ms instead of 2.67).
 using LinHalf = float2 (*)(bool, int, float, bool, bool, bool);
-template <bool STD, int NT>
-__device__ volatile LinHalf wide_half = lin_half<STD, WideWeights, NT>;
+template <bool STD, class S>
+__device__ volatile LinHalf wide_half = lin_half<STD, WideWeights, S>;
 
-template <bool STD, int NT>
-__global__ void __launch_bounds__(NT, 256 / NT) resident_kernel(const __grid_constant__ ResArgs p) {
+template <bool STD, class S>
+__global__ void __launch_bounds__(S::kThreads, 256 / S::kThreads) resident_kernel(const __grid_constant__ ResArgs p) {
   const int tid = threadIdx.x;
   ResCta& cta = res_cta();
   for (int task = blockIdx.x; task < p.n_tasks;) {
@@ -1283,17 +1302,18 @@ __global__ void __launch_bounds__(NT, 256 / NT) resident_kernel(const __grid_con
       max_window = max(max_window, o.window);
     }
     const bool mine = cb != nullptr;
-    res_word<NT>(kWordPar)[tid] = 0;
+    res_word<S>(kWordPar)[tid] = 0;
     if (tid == 0) {
       cta.slot = reinterpret_cast<char*>(p.scratch + p.slot * blockIdx.x);
       cta.guard = p.guard;
-      cta.rows8 = p.rows8;
+      cta.rows8 = max_window / 8;
+      cta.plane = 16u * lanes;
       cta.xs4 = 4u * res_pitch(lanes);
       cta.max_window = max_window;
     }
     if (tid < 16) cta.crc_tab[tid] = __ldg(p.xpow + kXpowSize + tid);
     __syncthreads();
-    res_window<NT>()[tid] = win;  // read by this thread alone
+    res_window<S>()[tid] = win;  // read by this thread alone
     bool passed = false;
     int used = p.max_iterations;
 
@@ -1309,21 +1329,21 @@ __global__ void __launch_bounds__(NT, 256 / NT) resident_kernel(const __grid_con
       if (pass != kPlain && !__syncthreads_or(run)) continue;
       const bool taken = run;
       if (pass != kWide) {
-        sys = res_inputs<STD, NT>(cb, p.llr, p.perm, pass == kPlain, from == 0);
+        sys = res_inputs<STD, S>(cb, p.llr, p.perm, pass == kPlain, from == 0);
         __syncthreads();
       }
       if (pass == kLog) {
-        if (run && from > 0) res_restore<NT>(from & 1);
+        if (run && from > 0) res_restore<S>(from & 1);
         __syncthreads();
       }
       if (pass == kPlain) {
-        int* const largest = res_word<NT>(kWordExt);
+        int* const largest = res_word<S>(kWordExt);
         largest[tid] = 0;
         __syncthreads();
         if (run) atomicMax(largest + lane0, __float_as_int(sys));
         __syncthreads();
         most = sys = __int_as_float(largest[lane0]);
-        q = __int_as_float(res_word<NT>(kWordPar)[lane0]);
+        q = __int_as_float(res_word<S>(kWordPar)[lane0]);
         __syncthreads();
         if (run && q > kMaxParity) {
           done_in = kLog;
@@ -1343,7 +1363,7 @@ __global__ void __launch_bounds__(NT, 256 / NT) resident_kernel(const __grid_con
             run = false;
           }
           if (!__syncthreads_or(run)) break;
-          const float2 c = lin_half<STD, Weights, NT>(run, half, scale, post_now, lower && p.early_stop, false);
+          const float2 c = lin_half<STD, Weights, S>(run, half, scale, post_now, lower && p.early_stop, false);
           if (run) {
             margin = c.x;
             most = sys + fabsf(scale) * c.y;
@@ -1356,7 +1376,7 @@ __global__ void __launch_bounds__(NT, 256 / NT) resident_kernel(const __grid_con
           const bool now = run && half >= from;
           if (!__syncthreads_or(now)) continue;
           const bool keep = margin < kNear || !(most <= kWideWeights - kNear);
-          const float2 c = wide_half<STD, NT>(now, half, scale, post_now, lower && p.early_stop, keep);
+          const float2 c = wide_half<STD, S>(now, half, scale, post_now, lower && p.early_stop, keep);
           if (now) {
             margin = most > kWideWeights ? -1.0f : c.x;
             most = sys + fabsf(scale) * c.y;
@@ -1369,30 +1389,30 @@ __global__ void __launch_bounds__(NT, 256 / NT) resident_kernel(const __grid_con
         } else {
           if (run && half >= from) {
             const float* d0 = p.llr + cb->llr;
-            if (lower) log_half<true, STD, NT>(d0, it, scale);
-            else log_half<false, STD, NT>(d0, it, scale);
+            if (lower) log_half<true, STD, S>(d0, it, scale);
+            else log_half<false, STD, S>(d0, it, scale);
           }
           __syncthreads();
-          if (run && half >= from) put_extrinsics<NT>(lower, post_now);
+          if (run && half >= from) put_extrinsics<S>(lower, post_now);
         }
         __syncthreads();
         if (post_now && p.early_stop) {
-          res_word<NT>(kWordSyn)[tid] = 0;
+          res_word<S>(kWordSyn)[tid] = 0;
           __syncthreads();
-          if (run && half >= from) res_crc<NT>(p.xpow, cb->filler);
+          if (run && half >= from) res_crc<S>(p.xpow, cb->filler);
           __syncthreads();
           if (run && half >= from) {
             used = it + 1;
-            passed = res_word<NT>(kWordSyn)[lane0] == 0;
+            passed = res_word<S>(kWordSyn)[lane0] == 0;
             // X goes from the posterior to the next iteration's input
-            if (!passed && !last_half) put_extrinsics<NT>(true, false);
+            if (!passed && !last_half) put_extrinsics<S>(true, false);
             run = !passed;
           }
           if (!__syncthreads_or(run)) break;
         }
       }
       const bool write = taken && done_in == pass;
-      res_outputs<NT>(write ? p.post + cb->out + (tid - lane0) * cb->window : nullptr,
+      res_outputs<S>(write ? p.post + cb->out + (tid - lane0) * cb->window : nullptr,
                       pass != kLog ? kLn2 : 1.0f);
       __syncthreads();
     }
