@@ -2,11 +2,11 @@
 //
 // One tc_decode call decodes any number of code blocks of any LTE sizes; every thread owns one
 // window of one code block.  The block-resident kernel (resident.cuh) runs all iterations in one
-// launch; layouts it cannot hold (very long windows in large batches, more than 256 windows per
-// block, more than 64 iterations) and the training schedule's short windows run as two launches per iteration (upper SISO over natural
-// order, lower SISO over QPP order) and, with early stop, one CRC24B launch.  This is the
-// replacement of the reference's Stage 1/2 host loops (lte_turbo_cuda.cu:1391-1540, 1719-1899),
-// batched over code blocks and correct for every K.
+// launch; plain windows below the default length (the training schedule's) and windows above 1024 steps
+// in batches of several waves run as two launches per iteration (upper SISO over natural order, lower
+// SISO over QPP order) and, with early stop, one CRC24B launch.  This is the replacement of the
+// reference's Stage 1/2 host loops (lte_turbo_cuda.cu:1391-1540, 1719-1899), batched over code blocks
+// and correct for every K.
 #include <cuda_runtime.h>
 
 #include <functional>
@@ -31,12 +31,13 @@ namespace tcb {
 
 namespace {
 
-// The kernel instances: CTAs of 32, 64, 96, 128 or 256 threads, and of 32 with a compact scratch slot.
+// The kernel instances: CTAs of 32, 64, 96 or 128 threads (a block has at most 48 windows there, pack_tasks),
+// and of 32 with a compact scratch slot.
 struct ResInstance {
   int threads;
   bool compact;
 };
-constexpr ResInstance kResInstances[] = {{32, true}, {32, false}, {64, false}, {96, false}, {128, false}, {256, false}};
+constexpr ResInstance kResInstances[] = {{32, true}, {32, false}, {64, false}, {96, false}, {128, false}};
 using ResKernel = void (*)(ResArgs);
 template <bool STD>
 ResKernel res_kernel_of(const ResInstance& i) {
@@ -45,8 +46,7 @@ ResKernel res_kernel_of(const ResInstance& i) {
     case 32: return resident_kernel<STD, Shape<32, false>>;
     case 64: return resident_kernel<STD, Shape<64, false>>;
     case 96: return resident_kernel<STD, Shape<96, false>>;
-    case 128: return resident_kernel<STD, Shape<128, false>>;
-    default: return resident_kernel<STD, Shape<256, false>>;
+    default: return resident_kernel<STD, Shape<128, false>>;
   }
 }
 ResKernel res_kernel(bool std3gpp, const ResInstance& i) {
@@ -342,12 +342,11 @@ Decoder::TuneChoice Decoder::autotune(const DecodeRequest& rq_in) {
                              {false, 176}, {false, 192}, {false, 224}, {false, 256},
                              {true, 192},  {true, 256},  {true, 320}};
   const int guard = rq_in.guard < 0 ? kDefaultGuard : rq_in.guard;
-  // Plain-schedule windows that fill whole waves: the smallest window (a multiple of 8, at
-  // least the guard) whose windows over all blocks fit in j resident waves of the SISO kernel
-  // (SMs x blocks per SM x threads per block), for j = 1 .. 4.  A launch with a partly filled
-  // last wave idles SMs for the length of a window (measured at 4096 x K=6144: window 136 = two
-  // full waves 2606 Mbit/s, window 128 = 2.07 waves 2457 Mbit/s); one wave of long windows
-  // spends the least on the guard warm-ups.
+  // And plain-schedule windows that fill whole waves of the launch-per-half-iteration kernel: the smallest
+  // window (a multiple of 8, at least the guard) whose windows over all blocks fit in j waves (SMs x blocks
+  // per SM x threads per block), for j = 1 .. 4.  Below 128 steps they run there, and are never the fastest;
+  // from 128 on they run in the block-resident kernel, whose waves are counted in tasks, and are no more than
+  // further lengths to try.
   const int64_t wave = static_cast<int64_t>(sm_count_) * kMinBlocks * kThreads;
   for (int j = 1; j <= 4; ++j) {
     for (int w = std::max(guard, kGroup); w <= 1024; w += kGroup) {
@@ -671,17 +670,18 @@ void Decoder::decode_now(const DecodeRequest& rq) {
 // launch-per-half-iteration kernels are the better (or only) way.
 void Decoder::pack_tasks(const DecodeRequest& rq, Layout& l) const {
   const size_t n = l.cbs.size();
-  if (rq.max_iterations > static_cast<uint32_t>(kMaxIterations) || l.max_windows > kResMaxThreads) return;
   // Windows asked for below the default length are the differentiable decoder's (64 steps).  The gradient
   // of its extrinsic scales is a sum whose terms cancel: the rounding of the forward pass alone moves it
   // by 1 to 3e-5 of its norm.  Its forward pass keeps the (m, s) kernels (1024 x K = 6144, 6 iterations,
   // forward and backward: 7.0 ms; 6.7 ms with this kernel as the forward pass), and so does the plain
-  // decode that has to equal it bit for bit.
+  // decode that has to equal it bit for bit.  From 128 steps on the two agree to rounding, and the plain
+  // decode is 2 to 3 times as fast as the (m, s) kernels.
   if (!rq.persistent && rq.window > 0 && rq.window < kDefaultWindow) return;
+  // That leaves 48 windows per block at most (the persistent layout has 32).
   // threads per CTA: one warp when every block fits in it; else the multiple of 32 up to 128 that
   // whole blocks of the largest window count fill best (48 windows of K = 6144 at 128 steps: two
   // blocks in 96), unless the batch is too small to give every SM a CTA of several blocks
-  l.threads = l.max_windows > 128 ? 256 : (l.max_windows + 31) / 32 * 32;
+  l.threads = (l.max_windows + 31) / 32 * 32;
   if (l.max_windows > 32 && n > 2 * static_cast<size_t>(sm_count_)) {
     double best = 0.0;
     for (int t = l.threads; t <= 128; t += 32) {
@@ -692,7 +692,7 @@ void Decoder::pack_tasks(const DecodeRequest& rq, Layout& l) const {
       }
     }
   }
-  size_t cap = res_x_bytes(32, 192) * static_cast<size_t>(l.threads / 32);  // 7 warps' worth per SM
+  size_t cap = res_x_bytes(32, 192) * static_cast<size_t>(l.threads / 32);  // 8 warps' worth per SM
   for (const DevCb& d : l.cbs) cap = std::max(cap, res_x_bytes(d.nwin, d.window));
   cap = std::min(cap, static_cast<size_t>(kResMaxX));
   // counting sort by block size, largest first

@@ -40,7 +40,6 @@
 namespace tcb {
 namespace {
 
-constexpr int kResMaxThreads = 256;
 constexpr int kResMaxX = 65536 - 256;             // bytes of X: its offsets are 16 bits
 constexpr int kResMaxSmem = 227 * 1024;
 constexpr uint64_t kWaitLimitNs = 1000000000ull;  // of a device-side wait: one second
