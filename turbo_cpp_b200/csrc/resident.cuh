@@ -5,8 +5,8 @@
 // extrinsic) stays in shared memory for the whole decode, in natural order, so neither SISO needs
 // an interleaved copy and no half-iteration waits for another CTA.  The streams that are only read
 // (parities, systematic) and the alpha checkpoints sit in a scratch slot per resident CTA, laid
-// out so that the lanes of a warp access consecutive words; the slots are reused from task to task
-// and stay in L2.
+// out so that the lanes of a warp access consecutive words; the slots are reused from task to task.
+// With all SMs full they are larger than L2 (246 MB at windows of 192) and are partly read from DRAM again.
 //
 // Arithmetic: the state metrics are kept as probabilities (float32, scaled by powers of two), not
 // as logarithms.  A trellis step of the 8 states is 16 multiply-adds and two ex2 for the branch
@@ -488,9 +488,8 @@ struct ResCta {
 extern __shared__ __align__(16) char res_smem[];
 constexpr int kResHead = (sizeof(ResCta) + 15) / 16 * 16;
 // Streams of the slot come through a ring in shared memory (cp.async, each thread its own
-// entries), because the slots of all resident CTAs together are about as large as L2: a group of
-// 8 steps is requested several groups before its use, which covers a DRAM access without holding
-// registers.  Stage: entries of 16 bytes per thread, [entry][thread].
+// entries), because the slots of all resident CTAs together are larger than L2: a group of 8 steps is
+// requested two groups before its use, which covers most of a DRAM access without holding registers.  Stage: entries of 16 bytes per thread, [entry][thread].
 constexpr int kStages = 2;
 constexpr int kEntries = 3;  // of a stage: 2 of parity, 1 of positions
 __host__ __device__ constexpr int res_ring_at(int nt) { return kResHead + 4 * nt; }

@@ -1,5 +1,6 @@
-// siso.cuh -- one window of one SISO half-iteration of the launch-per-half-iteration decoder
-// (windows too long for the block-resident one, the allocation-free entry point).
+// siso.cuh -- one window of one SISO half-iteration in the (m, s) form: the launch-per-half-iteration
+// decoder (plain windows below 128 steps, long windows in several waves, the allocation-free entry point),
+// the differentiable decoder's forward pass, and the block-resident decoder's last pass.
 //
 // A window [lo, hi) of a code block is owned by one thread, which keeps the 8 state metrics
 // in registers.  Its forward recursion starts `guard` steps before the window and its backward
