@@ -173,12 +173,12 @@ def measured_peaks():
         return 6650.0, "fallback"
 
 
-def ncu_traffic(schedule: str):
-    """DRAM bytes per trellis step of the SISO kernel from the committed ncu summary."""
+def ncu_traffic(schedule: str, window: int):
+    """DRAM bytes per trellis step of the resident kernel at K=6144 from the committed ncu summary."""
     path = os.path.join(ROOT, "profiles", "siso_dram_traffic.json")
     try:
         with open(path) as f:
-            return float(json.load(f)[schedule]["dram_bytes_per_step"])
+            return float(json.load(f)[f"{schedule}_{window}"]["dram_bytes_per_step"])
     except (OSError, KeyError, ValueError, TypeError):
         return None
 
@@ -767,7 +767,7 @@ def main():
     steps_per_launch = tm["trellis_steps"] / max(tm["siso_launches"], 1)
     achieved = FP32_PER_STEP * steps_per_launch / (avg_launch_ms / 1e3) / 1e9
     peak = props.multi_processor_count * FP32_PER_SM_CLK * sm_mhz * 1e6 / 1e9
-    traffic_per_step = ncu_traffic(schedule_name)
+    traffic_per_step = ncu_traffic(schedule_name, window)
     hbm_peak, hbm_src = measured_peaks()
     # algorithmic bytes of the launch: its share of the decode's 16 B per info bit
     alg_bytes_launch = steps_per_launch * BYTES_PER_BIT / (2 * it)
@@ -793,8 +793,8 @@ def main():
             "peak_source": f"{props.multi_processor_count} SMs x {FP32_PER_SM_CLK} FP32/clk x "
                            f"median sampled SM clock {sm_mhz:.0f} MHz (nominal issue rate)",
             "note": "achieved counts the recursions' own arithmetic once; with the windows' warm-ups, the "
-                    "recomputed alpha, branch weights and checks the kernel executes about 160 "
-                    "instructions per step, 94 on the FMA pipe, and instruction issue binds "
+                    "recomputed alpha, branch weights and checks the kernel executes about 129 "
+                    "instructions per step, 59 on the FMA pipe, and instruction issue binds "
                     "(profiles/resident_kernel_k6144x1036.md); no tensor cores (not a contraction); HBM "
                     "well below its peak (roofline_hbm)",
         },

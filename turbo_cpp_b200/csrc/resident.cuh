@@ -22,13 +22,12 @@
 //
 // The linear passes keep all LLRs in base-2 units (natural LLR * log2(e)).
 //
-// What bounds it: the issue slots of the SMs, at 2 warps per scheduler (about 126 instructions per step of a
+// What bounds it: the issue slots of the SMs, at 2 warps per scheduler (about 129 instructions per step of a
 // half-iteration, warm-ups included, 161 before most multiplications and multiply-adds went in pairs; the
 // (m, s) form has about 450).  One warp of 32 windows of 192 steps per CTA, because the shared memory of an
 // SM holds X of 8 of them (7 CTAs with rows of 33 words and a ring of 4 stages were 4 % slower).  4096
-// blocks of K = 6144, 8 iterations: 2.80 ms, 2.89 ms without the pairs, 8.0 ms with the (m, s) kernel that
-// this one replaced.  One block of K = 6144 from host memory: 0.43 ms (0.44, 1.08 ms); 20000 mixed blocks
-// with early stop: 6.2 ms (6.8, 14.3 ms).
+// blocks of K = 6144, 8 iterations: 2.69 ms, 8.0 ms with the (m, s) kernel that this one replaced.  One block
+// of K = 6144 from host memory: 0.42 ms (1.08 ms); 20000 mixed blocks with early stop: 5.9 ms (14.3 ms).
 #pragma once
 #include <cuda_runtime.h>
 
