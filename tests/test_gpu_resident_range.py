@@ -115,3 +115,37 @@ def test_restart_from_the_beginning(tc, decoder, oracle, iters, guard, std):
     ks = [512] * 300
     llr = std_code_blocks(tc, ks, 1.5, 37)[0] if std else awgn_blocks(tc, ks, 1.5, 37)[0]
     _compare(tc, decoder, oracle, ks, 3.0 * llr, iters, std=std, guard=guard)
+
+
+@pytest.mark.parametrize("std", [False, True])
+@pytest.mark.parametrize("persistent", [False, True])
+def test_infinite_llrs(tc, decoder, oracle, persistent, std):
+    """Known bits as infinite LLRs (systematic of either sign, parities known to be 0): weights of exactly 0,
+    which lose nothing.  Against 64 bits with 1e6 in their place; the known positions come back infinite."""
+    rng = np.random.default_rng(38)
+    ks = [40, 512, 1056, 6144, 104, 6144]
+    sent = np.sign(std_code_blocks(tc, ks, 40.0, 38)[0] if std else awgn_blocks(tc, ks, 40.0, 38)[0])
+    sigma2 = 1.5 / 10 ** 0.05
+    llr = (2 / sigma2 * (sent + np.sqrt(sigma2) * rng.normal(size=sent.size))).astype(np.float32)
+    known = np.zeros(llr.size, bool)
+    lo = 0
+    for k in ks:
+        known[lo + 3:lo + k:17] = True
+        for p in (1, 2):
+            known[lo + p * (k + 4) + 5:lo + p * (k + 4) + k:31] = True
+            known[lo + p * (k + 4):lo + p * (k + 4) + k] &= sent[lo + p * (k + 4):lo + p * (k + 4) + k] < 0
+        lo += 3 * (k + 4)
+    sched = tc.SCHEDULE_PERSISTENT if persistent else tc.SCHEDULE_PLAIN
+    conv = tc.CONVENTION_3GPP if std else tc.CONVENTION_REFERENCE
+    given = np.where(known, sent * np.inf, llr).astype(np.float32)
+    post, _, _ = decoder.decode(ks, given, None, tc.DecodeOptions(4, False, 0, 96, sched, convention=conv))
+    lo = po = 0
+    for k in ks:
+        x = np.where(known, sent * 1e6, llr)[lo:lo + 3 * (k + 4)]
+        ref = oracle.adj_vjp(k, x, [1.0] * 8, schedule_window(k, persistent), 96, std=std)[0]
+        got, at = post[po:po + k], known[lo:lo + k]
+        assert np.array_equal(got[at], sent[lo:lo + k][at] * np.inf), k
+        bar = np.maximum(1e-3 * np.maximum(np.abs(ref), 1.0), 2e-5 * np.abs(ref[~at]).max())
+        assert (np.abs(got - ref) <= bar)[~at].all(), k
+        lo += 3 * (k + 4)
+        po += k

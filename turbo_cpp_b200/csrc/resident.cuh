@@ -125,12 +125,14 @@ struct Shape {
 //   log2(smallest mass) - max |x| >= top + 13 - 150 + kKept.
 // That holds as long as it is metrics that lose, never weights (a lost weight counts relative to metrics
 // of up to 2^top), and as long as nothing grows again that was lost.  So, with q = log2 of the largest parity
-// weight or of its inverse:
+// weight or of its inverse (weights below 2^-kVoid left out, see the first point):
 // - While every weight is above 2^-126, |s| + q <= kPlainWeights for the largest |s|, the unlikely input's
 //   weight is one factor (the plain form).  Beyond that, or within kNear of the limit, the block changes to
-//   two factors of 2^(-|s| / 2) applied to the metrics one after the other (WideWeights), good for |s| up
-//   to kWideWeights.  The largest |s| is bounded by the systematic LLR's and the last extrinsic's maxima,
-//   which costs nothing per step.
+//   two factors of 2^(-|s| / 2) applied to the metrics one after the other (WideWeights).  They are 0 from
+//   252 bits on, where the product with a metric, below 2^(top + 15), is far below 2^-150 in any case; so is
+//   a parity weight below 2^-kVoid.  (Infinite LLRs of known bits are exact: weights of 0 that lose nothing.)
+//   The largest |s| is bounded by the systematic LLR's and the last extrinsic's maxima, which costs nothing
+//   per step.
 // - beta multiplies by the input weights first, the power of two of `weights` among them, and by the
 //   parity weight then, up to 2^q: the plain form leaves q bits less.  (The two-factor form applies the power
 //   of two behind the parity; the TS 36.212 code has one product per branch.)
@@ -143,13 +145,13 @@ struct Shape {
 // that passed were within 1.1e-5 max(|x + s|, 1 nat).  One factor throughout and neither deduction: off by up
 // to 18 bits.
 constexpr int kKept = 18;
-// A block within kNear of either limit of the two-factor form keeps what its half-iterations read, so that the
-// (m, s) pass can go on there (a store more per step); one that fails from further off starts again.
+// A block of the two-factor form that is within kNear of failing keeps what its half-iterations read, so that
+// the (m, s) pass can go on there (a store more per step); one that fails from further off starts again.
 constexpr float kNear = 40.0f;
 constexpr float kLost = 150.0f - 13.0f - kKept;
 constexpr float kPlainWeights = 126.0f;
-constexpr float kWideWeights = 250.0f;  // 2^(-|s| / 2) above 2^-126
-constexpr float kMaxParity = 76.0f;  // larger ones (of either sign) go to the (m, s) pass at once
+constexpr float kMaxParity = 76.0f;  // larger ones (of either sign, but for the void) go to the (m, s) pass at once
+constexpr float kVoid = 230.0f;      // 150 bits and those of the largest product of a metric and a weight
 constexpr int kTopMax = 60;
 // top of a block whose largest parity weight is 2^q: leaves the products of a step 18 bits of growth
 // below 2^126 (on ordinary channels alpha and beta grow by 4 or 5 each)
@@ -1089,13 +1091,14 @@ __device__ __noinline__ float res_inputs(const ResCb* cb, const float* llr, cons
       for (int r = 0; r < v.window; r += 4) {
         float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (r < v.len) x = *reinterpret_cast<const float4*>(row + 4 * r);
-        most = max3(max3(most, fabsf(x.x), fabsf(x.y)), fabsf(x.z), fabsf(x.w));
         x = make_float4(unit * x.x, unit * x.y, unit * x.z, unit * x.w);
+        const auto size = [&](float y) { return which != 0 && y < -kVoid ? 0.0f : fabsf(y); };
+        most = max3(max3(most, size(x.x), size(x.y)), size(x.z), size(x.w));
         if (exp_now) x = make_float4(ex2(x.x), ex2(x.y), ex2(x.z), ex2(x.w));
         m.st(m.record(which == 2, r >> 3) + (which == 0 ? m.sys() : 0) + m.half(r) + 16u * tid, x);
       }
-      if (which != 0) atomicMax(res_word<S>(kWordPar) + v.lane0, __float_as_int(unit * most));
-      else sys = unit * most;
+      if (which != 0) atomicMax(res_word<S>(kWordPar) + v.lane0, __float_as_int(most));
+      else sys = most;
     }
     __syncwarp();
   }
@@ -1371,11 +1374,10 @@ __global__ void __launch_bounds__(S::kThreads, 256 / S::kThreads) resident_kerne
         } else if (pass == kWide) {
           const bool now = run && half >= from;
           if (!__syncthreads_or(now)) continue;
-          const bool keep = margin < kNear || !(most <= kWideWeights - kNear);
+          const bool keep = margin < kNear;
           const float2 c = wide_half<STD, S>(now, half, scale, post_now, lower && p.early_stop, keep);
           if (now) {
-            margin = most > kWideWeights ? -1.0f : c.x;
-            most = sys + fabsf(scale) * c.y;
+            margin = c.x;
             if (!(margin >= 0.0f)) {
               done_in = kLog;
               from = keep ? half : 0;
