@@ -13,9 +13,9 @@
 // weights, where the (m, s) form of trellis.cuh needs 8 ex2 and about 85 instructions; the
 // extrinsic is one lg2 of each of two 4-term sums.  What limits it is float's exponent range: a
 // probability below 2^-149 becomes 0.  Each half-iteration checks, per block, that what was lost cannot
-// matter (kLost below).  A block whose LLRs are about to leave the range of one weight per input (126
-// bits) or whose checks come close goes on in a two-factor form of the same arithmetic, and from there,
-// if it has to, in the (m, s) form (siso.cuh), in passes of their own.  LLRs of ordinary channels stay
+// matter (kLost below).  A block whose LLRs leave the range of one weight per input (126 bits) or whose
+// checks come close goes on in a two-factor form of the same arithmetic, and from there, if it has to, in
+// the (m, s) form (siso.cuh), in passes of their own.  LLRs of ordinary channels stay
 // inside the linear range (extrinsics of about 120 to 170 bits, depending on the parities; eight
 // iterations at 1/3 reach 90 bits at 1 dB, 143 at 2.5 dB); blocks of rate 4/5 that fail their CRC may
 // leave it, scaled-up LLRs do.
@@ -126,13 +126,14 @@ struct Shape {
 // That holds as long as it is metrics that lose, never weights (a lost weight counts relative to metrics
 // of up to 2^top), and as long as nothing grows again that was lost.  So, with q = log2 of the largest parity
 // weight or of its inverse (weights below 2^-kVoid left out, see the first point):
-// - While every weight is above 2^-126, |s| + q <= kPlainWeights for the largest |s|, the unlikely input's
-//   weight is one factor (the plain form).  Beyond that, or within kNear of the limit, the block changes to
-//   two factors of 2^(-|s| / 2) applied to the metrics one after the other (WideWeights).  They are 0 from
-//   252 bits on, where the product with a metric, below 2^(top + 15), is far below 2^-150 in any case; so is
-//   a parity weight below 2^-kVoid.  (Infinite LLRs of known bits are exact: weights of 0 that lose nothing.)
-//   The largest |s| is bounded by the systematic LLR's and the last extrinsic's maxima, which costs nothing
-//   per step.
+// - While every weight is above 2^-126 the unlikely input's weight is one factor (the plain form).  A block
+//   in which one is not, which alpha finds out before X changes, or that is within kNearPlain of the limit
+//   changes to two factors of 2^(-|s| / 2) applied to the metrics one after the other (WideWeights).  They are
+//   0 from 252 bits on, where the product with a metric, below 2^(top + 15), is far below 2^-150 in any case;
+//   so is a parity weight below 2^-kVoid.  (Infinite LLRs of known bits are exact: weights of 0 that lose
+//   nothing.)  The two-factor form takes half as long again: the change comes as late as is safe (a bound of |s|
+//   from the systematic LLR's and the extrinsics' maxima instead of the weights themselves: 4096 blocks of K =
+//   6144 at 2 dB 3.5 ms instead of 3.0, 20000 of K = 512 at 3 dB 3.4 instead of 2.7).
 // - beta multiplies by the input weights first, the power of two of `weights` among them, and by the
 //   parity weight then, up to 2^q: the plain form leaves q bits less.  (The two-factor form applies the power
 //   of two behind the parity; the TS 36.212 code has one product per branch.)
@@ -148,8 +149,8 @@ constexpr int kKept = 18;
 // A block of the two-factor form that is within kNear of failing keeps what its half-iterations read, so that
 // the (m, s) pass can go on there (a store more per step); one that fails from further off starts again.
 constexpr float kNear = 40.0f;
+constexpr float kNearPlain = 30.0f;  // (24: some blocks fail all at once and start again, 512 transport blocks 7 % slower)
 constexpr float kLost = 150.0f - 13.0f - kKept;
-constexpr float kPlainWeights = 126.0f;
 constexpr float kMaxParity = 76.0f;  // larger ones (of either sign, but for the void) go to the (m, s) pass at once
 constexpr float kVoid = 230.0f;      // 150 bits and those of the largest product of a metric and a weight
 constexpr int kTopMax = 60;
@@ -159,7 +160,12 @@ __device__ __forceinline__ int res_top(float q) {
   return min(kTopMax, static_cast<int>(0.5f * (108.0f - fminf(q, kMaxParity))));
 }
 
-// min(x, y), max(x, y, z), NaN if any is
+// min(x, y, z) of what is not NaN; min(x, y), max(x, y, z), NaN if any is
+__device__ __forceinline__ float min3(float x, float y, float z) {
+  float r;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(x), "f"(y), "f"(z));
+  return r;
+}
 __device__ __forceinline__ float min_nan(float x, float y) {
   float r;
   asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(x), "f"(y));
@@ -178,6 +184,7 @@ __device__ __forceinline__ float max3_nan(float x, float y, float z) {
 struct Weights {
   static constexpr bool kWide = false;
   float a1, a0, b;
+  float x;  // the smaller of a1, a0
 };
 __device__ __forceinline__ float weight_scale(float b) {
   return __int_as_float(0x7f000000 - (__float_as_int(fmaxf(b, 1.0f)) & 0x7f800000));
@@ -185,7 +192,7 @@ __device__ __forceinline__ float weight_scale(float b) {
 __device__ __forceinline__ void weights(float s, float b, Weights& w) {
   const float y = weight_scale(b);
   const float x = ex2(-fabsf(s)) * y;
-  w = Weights{s < 0.0f ? x : y, s < 0.0f ? y : x, b};
+  w = Weights{s < 0.0f ? x : y, s < 0.0f ? y : x, b, x};
 }
 // The same in the two-factor form: input 1 / input 0 are c1^2 y / c0^2 y, y the power of two and c of the
 // unlikely input 2^(-|s| / 2).
@@ -392,6 +399,16 @@ __device__ __forceinline__ void beta_next(int step, float (&be)[8], const Weight
 #pragma unroll
     for (int n = 0; n < 8; ++n) be[n] = t[n];
   }
+}
+// The smallest weight of two steps (the TS 36.212 code: or product of weights) and `least`.
+template <bool STD>
+__device__ __forceinline__ float least_of(float least, const Weights& v, const Weights& w) {
+  least = min3(least, v.x, w.x);
+  return STD ? min3(least, v.x * v.b, w.x * w.b) : least;
+}
+template <bool STD>
+__device__ __forceinline__ float least_of(float least, const WideWeights&, const WideWeights&) {
+  return least;
 }
 // The mass of all paths from the sums of alpha beta over the branches with input 1 and 0.
 __device__ __forceinline__ float mass_of(const Weights& w, float s1, float s0) { return fmaf(w.a1, s1, w.a0 * s0); }
@@ -661,10 +678,11 @@ struct Ring {
 
 // One SISO half-iteration of one window in the linear domain, first part: everything that reads
 // other windows' positions of X.  Leaves the alpha checkpoints and the next window's alpha seed,
-// and beta at the window's end in `be`; `fall` becomes the largest rescaling of the window's alpha.
+// and beta at the window's end in `be`; `fall` becomes the largest rescaling of the window's alpha, `least`
+// (plain form) its steps' smallest weight.
 template <bool STD, class W, class S>
 __device__ __forceinline__ void lin_read(const ResWin& v, const Slot<S>& m, const int it, const bool lower,
-                                         float (&be)[8], float& fall) {
+                                         float (&be)[8], float& fall, float& least) {
   const uint32_t kPlane = m.plane, kRecord = 5 * m.plane;
   const char* const X = res_x<S>();
   const int tid = v.tid, G = v.guard;
@@ -715,12 +733,17 @@ __device__ __forceinline__ void lin_read(const ResWin& v, const Slot<S>& m, cons
       }
       request(ring.at);
       ring.advance();
+      float low = 1.0f;
 #pragma unroll
-      for (int t = 0; t < 8; ++t) {
-        W w;
-        weights(s[t], b[t], w);
-        alpha_next<STD>(t, al, w);
+      for (int t = 0; t < 8; t += 2) {
+        W w[2];
+        weights(s[t], b[t], w[0]);
+        weights(s[t + 1], b[t + 1], w[1]);
+        low = least_of<STD>(low, w[0], w[1]);
+        alpha_next<STD>(t, al, w[0]);
+        alpha_next<STD>(t + 1, al, w[1]);
       }
+      if (j >= 0) least = fminf(least, low);
     }
   }
   const int tail_at = v.k - (v.lo + v.len);  // steps of the block behind the window
@@ -907,16 +930,29 @@ __device__ __forceinline__ float2 lin_write(const ResWin& v, const Slot<S>& m, c
 }
 
 // A half-iteration of the CTA's blocks in the linear domain; `run`: this thread's window takes part.
-// Returns the bits by which its block passed the checks (negative: it did not) and its largest extrinsic.
+// Returns the bits by which its block passed the checks (negative: it did not), and whether it ran: in the
+// plain form a block with a weight below 2^-126 is left as it was (below 0).
 template <bool STD, class W, class S>
-__device__ __noinline__ float2 lin_half(const bool run, const int half, const float scale, const bool post,
+__device__ __noinline__ float2 lin_half(bool run, const int half, const float scale, const bool post,
                                         const bool keep_ext, const bool keep) {
   const ResWin v = res_win<S>();
   const Slot<S> m;
   const bool lower = half & 1;
-  float be[8], fall = 1.0f;
-  if (run) lin_read<STD, W, S>(v, m, half >> 1, lower, be, fall);
+  float be[8], fall = 1.0f, least = 1.0f;
+  if (run) lin_read<STD, W, S>(v, m, half >> 1, lower, be, fall, least);
   __syncthreads();  // every window has read X (and left its seeds and checkpoints)
+  float ran = 1.0f;
+  if constexpr (!W::kWide) {
+    res_word<S>(kWordMass)[threadIdx.x] = 0x3f800000;
+    __syncthreads();
+    if (run) atomicMin(res_word<S>(kWordMass) + v.lane0, __float_as_int(least));
+    __syncthreads();
+    if (__int_as_float(res_word<S>(kWordMass)[v.lane0]) < 0x1p-126f) {
+      ran = -1.0f;
+      run = false;
+    }
+    __syncthreads();  // (the ring is in use again)
+  }
   float2 c = make_float2(0.0f, 0.0f);
   if (run) c = lin_write<STD, W, S>(v, m, half >> 1, lower, be, scale, post, keep_ext, keep);
   __syncthreads();
@@ -934,7 +970,7 @@ __device__ __noinline__ float2 lin_half(const bool run, const int half, const fl
   const float lost = !STD && !W::kWide ? word(kWordPar) : 0.0f;  // by the plain form's beta
   return make_float2(lg2(word(kWordMass)) - word(kWordExt) - (static_cast<float>(v.top) - kLost) - lost -
                          fmaxf(lg2(word(kWordFall)) - static_cast<float>(kKept), 0.0f),
-                     word(kWordExt));
+                     ran);
 }
 
 // The extrinsics in the checkpoint planes into X: added to Ls (the other SISO's input), or (post)
@@ -1029,10 +1065,9 @@ __device__ __forceinline__ void res_stage_rows(const ResWin& v, const void* src,
 // that goes on keeps the seeds of the half-iterations before).
 // Each warp stages its windows' rows through shared memory (where X and the ring will be; a row
 // pitch of an odd number of 16-byte words keeps both sides free of bank conflicts).
-// Returns the window's largest systematic |LLR|.
 template <bool STD, class S>
-__device__ __noinline__ float res_inputs(const ResCb* cb, const float* llr, const uint16_t* perm,
-                                         const bool linear, const bool start) {
+__device__ __noinline__ void res_inputs(const ResCb* cb, const float* llr, const uint16_t* perm,
+                                        const bool linear, const bool start) {
   const Slot<S> m;
   const float unit = linear ? kLog2e : 1.0f;
   const int tid = threadIdx.x;
@@ -1077,7 +1112,6 @@ __device__ __noinline__ float res_inputs(const ResCb* cb, const float* llr, cons
     __syncwarp();
   }
   const int pitch = 4 * W + 16;
-  float sys = 0.0f;
 #pragma unroll 1
   for (int st = 0; st < 3; ++st) {  // parity 1, parity 2, systematic
     const int which = st == 2 ? 0 : st + 1;
@@ -1092,13 +1126,12 @@ __device__ __noinline__ float res_inputs(const ResCb* cb, const float* llr, cons
         float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (r < v.len) x = *reinterpret_cast<const float4*>(row + 4 * r);
         x = make_float4(unit * x.x, unit * x.y, unit * x.z, unit * x.w);
-        const auto size = [&](float y) { return which != 0 && y < -kVoid ? 0.0f : fabsf(y); };
+        const auto size = [](float y) { return y < -kVoid ? 0.0f : fabsf(y); };
         most = max3(max3(most, size(x.x), size(x.y)), size(x.z), size(x.w));
         if (exp_now) x = make_float4(ex2(x.x), ex2(x.y), ex2(x.z), ex2(x.w));
         m.st(m.record(which == 2, r >> 3) + (which == 0 ? m.sys() : 0) + m.half(r) + 16u * tid, x);
       }
       if (which != 0) atomicMax(res_word<S>(kWordPar) + v.lane0, __float_as_int(most));
-      else sys = most;
     }
     __syncwarp();
   }
@@ -1125,7 +1158,7 @@ __device__ __noinline__ float res_inputs(const ResCb* cb, const float* llr, cons
     }
   }
   __syncthreads();
-  if (!mine) return 0.0f;
+  if (!mine) return;
 #pragma unroll 1
   for (int r0 = 0; r0 < v.window; r0 += 32) {
     uint4 q[4];
@@ -1155,7 +1188,6 @@ __device__ __noinline__ float res_inputs(const ResCb* cb, const float* llr, cons
       m.st8(m.tail(lower) + 16u * tid, tb);
     }
   }
-  return sys;
 }
 
 // This window's part of its block's CRC24B syndrome of the hard decisions [filler, K)
@@ -1321,14 +1353,13 @@ __global__ void __launch_bounds__(S::kThreads, 256 / S::kThreads) resident_kerne
     // block ends in, `from` the half-iteration where that pass takes over.
     int done_in = kPlain, from = 0;
     float margin = 1000.0f;  // of the block's checks in the last half-iteration
-    float q = 0.0f, sys = 0.0f, most = 0.0f;  // its largest parity and systematic LLR, a bound of |X|
 #pragma unroll 1
     for (int pass = kPlain; pass <= kLog && p.max_iterations > 0; ++pass) {
       bool run = mine && done_in == pass;
       if (pass != kPlain && !__syncthreads_or(run)) continue;
       const bool taken = run;
       if (pass != kWide) {
-        sys = res_inputs<STD, S>(cb, p.llr, p.perm, pass == kPlain, from == 0);
+        res_inputs<STD, S>(cb, p.llr, p.perm, pass == kPlain, from == 0);
         __syncthreads();
       }
       if (pass == kLog) {
@@ -1336,15 +1367,8 @@ __global__ void __launch_bounds__(S::kThreads, 256 / S::kThreads) resident_kerne
         __syncthreads();
       }
       if (pass == kPlain) {
-        int* const largest = res_word<S>(kWordExt);
-        largest[tid] = 0;
-        __syncthreads();
-        if (run) atomicMax(largest + lane0, __float_as_int(sys));
-        __syncthreads();
-        most = sys = __int_as_float(largest[lane0]);
-        q = __int_as_float(res_word<S>(kWordPar)[lane0]);
-        __syncthreads();
-        if (run && q > kMaxParity) {
+        const bool outside = run && __int_as_float(res_word<S>(kWordPar)[lane0]) > kMaxParity;
+        if (outside) {
           done_in = kLog;
           run = false;
         }
@@ -1356,16 +1380,19 @@ __global__ void __launch_bounds__(S::kThreads, 256 / S::kThreads) resident_kerne
         const bool post_now = lower && (p.early_stop || last_half);
         const float scale = __ldg(p.scale + half);
         if (pass == kPlain) {
-          if (run && (margin < kNear || !(most + q <= kPlainWeights))) {
+          if (run && margin < kNearPlain) {
             done_in = kWide;
             from = half;
             run = false;
           }
           if (!__syncthreads_or(run)) break;
           const float2 c = lin_half<STD, Weights, S>(run, half, scale, post_now, lower && p.early_stop, false);
-          if (run) {
+          if (run && c.y < 0.0f) {
+            done_in = kWide;
+            from = half;
+            run = false;
+          } else if (run) {
             margin = c.x;
-            most = sys + fabsf(scale) * c.y;
             if (!(margin >= 0.0f)) {
               done_in = kLog;
               run = false;
