@@ -793,7 +793,7 @@ def main():
             "peak_source": f"{props.multi_processor_count} SMs x {FP32_PER_SM_CLK} FP32/clk x "
                            f"median sampled SM clock {sm_mhz:.0f} MHz (nominal issue rate)",
             "note": "achieved counts the recursions' own arithmetic once; with the windows' warm-ups, the "
-                    "recomputed alpha, branch weights and checks the kernel executes about 129 "
+                    "recomputed alpha, branch weights and checks the kernel executes about 131 "
                     "instructions per step, 59 on the FMA pipe, and instruction issue binds "
                     "(profiles/resident_kernel_k6144x1036.md); no tensor cores (not a contraction); HBM "
                     "well below its peak (roofline_hbm)",

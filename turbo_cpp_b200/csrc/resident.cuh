@@ -22,7 +22,7 @@
 //
 // The linear passes keep all LLRs in base-2 units (natural LLR * log2(e)).
 //
-// What bounds it: the issue slots of the SMs, at 2 warps per scheduler (about 129 instructions per step of a
+// What bounds it: the issue slots of the SMs, at 2 warps per scheduler (about 131 instructions per step of a
 // half-iteration, warm-ups included, 161 before most multiplications and multiply-adds went in pairs; the
 // (m, s) form has about 450).  One warp of 32 windows of 192 steps per CTA, because the shared memory of an
 // SM holds X of 8 of them (7 CTAs with rows of 33 words and a ring of 4 stages were 4 % slower).  4096
